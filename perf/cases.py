@@ -3,7 +3,7 @@
 `listed()` names twelve fixed cases, `draw(rng)` gives further ones of the same ranges.  A case is
 a dict of plain values; `prepare` makes what a program holds before the call, `run` is one pass,
 `work` the bytes and operations a pass cannot do without, `tolerance` what another correct
-implementation at the same precision may differ by.
+implementation at the same precision may differ by, `exact` the results in 64 bits.
 
 Kinds of case:
   fwd    attention forward without gradients: inference over a whole sequence (prefill, encoders),
@@ -230,6 +230,80 @@ def run(state):
     o = _attention(state)
     dq, dk, dv = torch.autograd.grad(o, (state["q"], state["k"], state["v"]), state["grad_out"])
     return o, dq, dk, dv
+
+
+def _exact_lion(case, seed):
+    state = _prepare_lion(case, seed)
+    opt = state["opt"]
+    lr, wd, (b1, b2) = case["lr"], case["weight_decay"], (0.9, 0.99)
+    p_out, m_out = state["params"].double(), state["momentum"].double()
+    at = 0
+    for p in opt.param_groups[0]["params"]:
+        n = p.numel()
+        g = p.grad.reshape(-1).double()
+        pn, mn = p_out[at:at + n], m_out[at:at + n]
+        pn.mul_(1 - lr * wd).sub_((mn * b1 + g * (1 - b1)).sign_(), alpha=lr)
+        mn.mul_(b2).add_(g, alpha=1 - b2)
+        at += (n + 255) // 256 * 256
+    return p_out, m_out
+
+
+def _exact_head(q, k, v, bias, causal, grad_out):
+    """One head in 64 bits, a slab of query rows at a time: (o,) or (o, dq, dk, dv)."""
+    sq, d = q.shape
+    sk = k.shape[0]
+    q, k, v = q.double(), k.double(), v.double()
+    o = torch.empty_like(q)
+    dq, dk, dv = torch.empty_like(q), torch.zeros_like(k), torch.zeros_like(v)
+    scale = 1.0 / math.sqrt(d)
+    rows = max(64, (1 << 26) // sk)
+    for r in range(0, sq, rows):
+        e = min(sq, r + rows)
+        keys = min(sk, e) if causal else sk
+        s = (q[r:e] @ k[:keys].T) * scale
+        if bias is not None:
+            s += (bias[r:e, :keys] if bias.shape[0] > 1 else bias[:, :keys]).double()
+        if causal:
+            above = torch.arange(keys, device=q.device)[None, :] > torch.arange(r, e, device=q.device)[:, None]
+            s.masked_fill_(above, float("-inf"))
+        p = torch.softmax(s, dim=-1)
+        o[r:e] = p @ v[:keys]
+        if grad_out is not None:
+            g = grad_out[r:e].double()
+            ds = p * (g @ v[:keys].T - (g * o[r:e]).sum(-1, keepdim=True))
+            dq[r:e] = (ds @ k[:keys]) * scale
+            dk[:keys] += (ds.T @ q[r:e]) * scale
+            dv[:keys] += p.T @ g
+    return (o,) if grad_out is None else (o, dq, dk, dv)
+
+
+def exact(case, seed):
+    """The outputs of the first pass in 64 bits.  None with dropout (the mask is the framework's own)."""
+    if case["kind"] == "lion":
+        return _exact_lion(case, seed)
+    if case["dropout"] > 0:
+        return None
+    state = _prepare_attn(case, seed)
+    bshd, h, bias = state["bshd"], case["h"], state["bias"]
+
+    def heads(t):
+        return t.detach().transpose(1, 2) if bshd else t.detach()
+
+    q, k, v = heads(state["q"]), heads(state["k"]), heads(state["v"])
+    grad_out = heads(state["grad_out"]) if "grad_out" in state else None
+    outs = [torch.zeros(t.shape, dtype=torch.float64, device=t.device)
+            for t in ((q,) if grad_out is None else (q, q, k, v))]
+    for b in range(case["b"]):
+        for i in range(h):
+            j = i % k.shape[1]
+            one = None if bias is None else bias[b % bias.shape[0], i % bias.shape[1]]
+            got = _exact_head(q[b, i], k[b, j], v[b, j], one, case["causal"],
+                              None if grad_out is None else grad_out[b, i])
+            for out, x, at in zip(outs, got, (i, i, j, j)):
+                out[b, at] += x  # a shared key/value head collects its gradient from every query head
+    if bshd:
+        outs = [t.transpose(1, 2).contiguous() for t in outs]
+    return outs[0] if grad_out is None else tuple(outs)
 
 
 def _fwd_flops(case):
