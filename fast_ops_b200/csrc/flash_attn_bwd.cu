@@ -81,9 +81,9 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
                const CUtensorMap& tdq, const fo::AttnBwdParams& prm, cudaStream_t stream) {
   dim3 grid((prm.Sk + fo::kBlockN - 1) / fo::kBlockN, prm.B * prm.H);
   auto kernel = fo::attn_bwd_kernel<D, kBf16, kExt>;
-  constexpr int smem = fo::BwdConfig<D>::kSmemBytes;
+  constexpr int smem = fo::BwdConfig<D, kExt>::kSmemBytes;
   FO_CUDA_CHECK((fo::ensure_dynamic_smem<fo::attn_bwd_kernel<D, kBf16, kExt>>(smem, prm.device)));
-  kernel<<<grid, 512, smem, stream>>>(tq, tk, tv, tdo, tdq, prm);
+  kernel<<<grid, fo::BwdConfig<D, kExt>::kThreads, smem, stream>>>(tq, tk, tv, tdo, tdq, prm);
   fo::g_launch_count.fetch_add(1, std::memory_order_relaxed);
   FO_CUDA_CHECK(cudaGetLastError());
   return FO_OK;
@@ -187,7 +187,8 @@ static int attn_bwd_impl(const void* q, const void* k, const void* v, const void
   const bool ext = ex != nullptr && (ex->bias != nullptr || ex->dropout);
   if (ext) prm.ex = *ex;
   int rc;
-  const int mode = ext ? ((prm.ex.bias != nullptr ? 1 : 0) | (prm.ex.dropout ? 2 : 0)) : 0;
+  const int bias_mode = !ext || prm.ex.bias == nullptr ? 0 : prm.ex.bias_stride_q == 0 ? fo::kBwdVecBias : fo::kBwdMatBias;
+  const int mode = bias_mode | (ext && prm.ex.dropout ? fo::kBwdDropout : 0);
 #define FO_BWD_MODE(M)                                                                                     \
   case M:                                                                                                  \
     if (Dk == 128) rc = bf16 ? launch_bwd<128, true, M>(tq, tk, tv, tdo, tdq, prm, s) : launch_bwd<128, false, M>(tq, tk, tv, tdo, tdq, prm, s); \
@@ -197,8 +198,10 @@ static int attn_bwd_impl(const void* q, const void* k, const void* v, const void
     FO_BWD_MODE(0)
     FO_BWD_MODE(1)
     FO_BWD_MODE(2)
-    default:
     FO_BWD_MODE(3)
+    FO_BWD_MODE(4)
+    default:
+    FO_BWD_MODE(6)
   }
 #undef FO_BWD_MODE
   if (rc) return rc;
