@@ -10,6 +10,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "flash_attn_decode.cuh"
 #include "flash_attn_simple.cuh"
 #include "flash_attn_ws.cuh"
 #include "flash_attn_ws64.cuh"
@@ -215,6 +216,45 @@ int make_attn_extras(AttnExtras* ex, const void* bias, const int64_t* bias_strid
 
 }  // namespace fo
 
+// Launches the split-key kernel; strides are those check_layout returned, in elements.
+static int decode(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H, int Sk, int D,
+                  const int64_t qs[3], const int64_t ks[3], const int64_t vs[3], const int64_t os[3], bool kv_bcast,
+                  int dtype, float softmax_scale, const int* status, int num_sms, int device, cudaStream_t stream) {
+  fo::DecodeParams prm;
+  prm.q = static_cast<const uint16_t*>(q);
+  prm.k = static_cast<const uint16_t*>(k);
+  prm.v = static_cast<const uint16_t*>(v);
+  prm.o = static_cast<uint16_t*>(o);
+  prm.lse = lse;
+  prm.q_stride_b = qs[0];
+  prm.q_stride_h = qs[1];
+  prm.k_stride_b = ks[0];
+  prm.k_stride_h = kv_bcast ? 0 : ks[1];
+  prm.k_stride_s = ks[2];
+  prm.v_stride_b = vs[0];
+  prm.v_stride_h = kv_bcast ? 0 : vs[1];
+  prm.v_stride_s = vs[2];
+  prm.o_stride_b = os[0];
+  prm.o_stride_h = os[1];
+  prm.H = H;
+  prm.Sk = Sk;
+  prm.d_real = D;
+  prm.scale_log2 = softmax_scale * 1.4426950408889634f;
+  prm.device_status = status;
+  const bool bf16 = dtype == FO_BF16;
+  // Heads that share K and V go four to a CTA, so that the shared tensors cross L2 a quarter as often.
+#define FO_DECODE(DK, HEADS)                                                                 \
+  return bf16 ? fo::launch_decode<DK, true, HEADS>(prm, B, num_sms, device, stream)          \
+              : fo::launch_decode<DK, false, HEADS>(prm, B, num_sms, device, stream)
+  if (D <= 64) {
+    if (kv_bcast) FO_DECODE(64, 4);
+    FO_DECODE(64, 1);
+  }
+  if (kv_bcast) FO_DECODE(128, 4);
+  FO_DECODE(128, 1);
+#undef FO_DECODE
+}
+
 static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, float* lse,
                          int B, int H, int Sq, int Sk, int D,
                          const int64_t q_strides[3], const int64_t k_strides[3],
@@ -239,15 +279,30 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   int* status = fo::device_status_ptr(device);
   if (!status) return fo::fail(FO_ERR_CUDA, "cannot resolve the status word of device %d", device);
 
-  CUtensorMap tq, tk, tv;
-  if (int rc = make_tensor_map(&tq, q, dtype, B, H, Sq, D, q_strides, "q")) return rc;
   // Multi-query attention: K and V expanded over the head dimension with stride 0 (one shared
   // head, as the reference's tests build it, tests/test_flash_attention_triton.py:71-73) are
   // described to TMA as single-head tensors and every query head reads head 0.
   const bool kv_bcast = H > 1 && k_strides[1] == 0 && v_strides[1] == 0;
-  FO_REQUIRE(kv_bcast || H == 1 || (k_strides[1] != 0 && v_strides[1] != 0),
-             "k and v must both have a head stride, or both be expanded with head stride 0");
+  const bool kv_same = kv_bcast || H == 1 || (k_strides[1] != 0 && v_strides[1] != 0);
   const int Hkv = kv_bcast ? 1 : H;
+  const bool ext = ex != nullptr && (ex->bias != nullptr || ex->dropout);
+  const DeviceInfo* info = device_info(device);
+  if (!info) return fo::fail(FO_ERR_CUDA, "cannot look up device %d", device);
+  AttnImpl impl = static_cast<AttnImpl>(fo::g_attn_options.impl.load(std::memory_order_relaxed));
+  if (impl == AttnImpl::kAuto && Sq == 1 && !causal && !ext) {
+    // One query row per head: the split-key kernel.  (With a causal mask only key 0 is visible.)
+    int64_t qs[3], ks[3], vs[3];
+    if (int rc = fo::check_layout(q, B, H, Sq, D, q_strides, "q", qs)) return rc;
+    FO_REQUIRE(kv_same, "k and v must both have a head stride, or both be expanded with head stride 0");
+    if (int rc = fo::check_layout(k, B, Hkv, Sk, D, k_strides, "k", ks)) return rc;
+    if (int rc = fo::check_layout(v, B, Hkv, Sk, D, v_strides, "v", vs)) return rc;
+    return decode(q, k, v, o, lse, B, H, Sk, D, qs, ks, vs, o_strides, kv_bcast, dtype, softmax_scale, status, info->num_sms,
+                  device, static_cast<cudaStream_t>(stream));
+  }
+
+  CUtensorMap tq, tk, tv;
+  if (int rc = make_tensor_map(&tq, q, dtype, B, H, Sq, D, q_strides, "q")) return rc;
+  FO_REQUIRE(kv_same, "k and v must both have a head stride, or both be expanded with head stride 0");
   if (int rc = make_tensor_map(&tk, k, dtype, B, Hkv, Sk, D, k_strides, "k")) return rc;
   if (int rc = make_tensor_map(&tv, v, dtype, B, Hkv, Sk, D, v_strides, "v")) return rc;
 
@@ -270,13 +325,10 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   prm.kv_head_bcast = kv_bcast ? 1 : 0;
   prm.ping_pong = fo::g_attn_options.ping_pong.load(std::memory_order_relaxed);
   prm.device = device;
-  const DeviceInfo* info = device_info(device);
-  if (!info) return fo::fail(FO_ERR_CUDA, "cannot look up device %d", device);
   prm.num_sms = info->num_sms;
   prm.sched = info->sched + 2 * (g_sched_next.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
   std::memset(&prm.ex, 0, sizeof(prm.ex));
   prm.ex.drop_rescale = 1.f;
-  const bool ext = ex != nullptr && (ex->bias != nullptr || ex->dropout);
   if (ext) prm.ex = *ex;
   {
     // as many heads per group as keep their K and V (2 * Sk * D * 2 bytes each) within about a
@@ -292,7 +344,6 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool bf16 = dtype == FO_BF16;
-  AttnImpl impl = static_cast<AttnImpl>(fo::g_attn_options.impl.load(std::memory_order_relaxed));
   if (impl == AttnImpl::kAuto) {
     // The 64-key-step kernel is the faster one at every shape measured (same box, hot loop, bf16
     // causal: S=16384 1.11 against 1.02 PFLOP/s, S=4096 0.98 against 0.82, GPT-2-small shape

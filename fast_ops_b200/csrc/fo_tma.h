@@ -30,6 +30,23 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// What every 16-bit attention tensor must satisfy: a 16-byte base, positive strides that are
+// multiples of 8 elements, rows that do not overlap.  A dimension of extent 1 never uses its
+// stride; it gets a harmless one.  Returns the strides (batch, head, row) in `out`.
+inline int check_layout(const void* base, int B, int H, int S, int D, const int64_t strides[3], const char* name,
+                        int64_t out[3]) {
+  FO_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "%s must be 16-byte aligned", name);
+  const int64_t sb = B > 1 ? strides[0] : static_cast<int64_t>(H) * S * D;
+  const int64_t sh = H > 1 ? strides[1] : static_cast<int64_t>(S) * D;
+  const int64_t ss = S > 1 ? strides[2] : D;
+  FO_REQUIRE(sb > 0 && sh > 0 && ss >= D, "%s: strides must be positive and rows must not overlap", name);
+  FO_REQUIRE(sb % 8 == 0 && sh % 8 == 0 && ss % 8 == 0, "%s: strides must be multiples of 8 elements", name);
+  out[0] = sb;
+  out[1] = sh;
+  out[2] = ss;
+  return FO_OK;
+}
+
 // Tensor map over a (B, H, S, D) tensor with element strides (sb, sh, ss, 1): dimensions are
 // listed innermost first, the box is one [box_rows x 64 columns] swizzled tile (128 rows, or 64
 // for the half tiles of the short-sequence kernel), and reads past S are filled with zeros.
@@ -37,13 +54,9 @@ inline int encode_tensor_map(CUtensorMap* map, const void* base, int dtype, int 
                              const int64_t strides[3], const char* name, int box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fo::fail(FO_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  FO_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "%s must be 16-byte aligned", name);
-  // A dimension of extent 1 never uses its stride; give it a harmless one.
-  int64_t sb = B > 1 ? strides[0] : static_cast<int64_t>(H) * S * D;
-  int64_t sh = H > 1 ? strides[1] : static_cast<int64_t>(S) * D;
-  int64_t ss = S > 1 ? strides[2] : D;
-  FO_REQUIRE(sb > 0 && sh > 0 && ss >= D, "%s: strides must be positive and rows must not overlap", name);
-  FO_REQUIRE(sb % 8 == 0 && sh % 8 == 0 && ss % 8 == 0, "%s: strides must be multiples of 8 elements", name);
+  int64_t st[3];
+  if (int rc = check_layout(base, B, H, S, D, strides, name, st)) return rc;
+  const int64_t sb = st[0], sh = st[1], ss = st[2];
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(H),
                               static_cast<cuuint64_t>(B)};
   const cuuint64_t gstrides[3] = {static_cast<cuuint64_t>(ss) * 2, static_cast<cuuint64_t>(sh) * 2,

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import oracle
+from fast_ops_b200.flash_attention import flash_attention_forward
 from test_gpu_5_attention_bias_dropout import check, run_case
 
 pytestmark = pytest.mark.gpu
@@ -31,3 +32,59 @@ def test_backward_bias_and_dropout_variants(cuda_device, Sq, Sk, causal, D, code
     keep = oracle.dropout_mask(p, B, H, Sq, Sk, *rng) if p > 0 else None
     out, _, dq, dk, dv = oracle.attention_ex(q, k, v, bias=bias, keep_mask=keep, dropout_p=p, causal=causal, dout=dout)
     check(got, same, (out, dq, dk, dv), f"D={D} {code} p={p}")
+
+
+@pytest.mark.parametrize("B,H,Sk,D,dtype,kv_heads,layout", [
+    (1, 1, 1, 64, torch.bfloat16, 1, "bhsd"), (2, 3, 7, 128, torch.float16, 3, "bhsd"),
+    (1, 2, 255, 40, torch.bfloat16, 2, "bshd"), (3, 5, 511, 128, torch.bfloat16, 1, "bhsd"),
+    (1, 4, 513, 64, torch.float16, 1, "bshd"), (2, 2, 1024, 8, torch.float16, 2, "bhsd"),
+    (1, 8, 4099, 128, torch.bfloat16, 8, "bshd"), (1, 6, 3000, 96, torch.float16, 1, "bhsd"),
+    (2, 3, 2049, 80, torch.bfloat16, 3, "bhsd"), (40, 8, 600, 64, torch.bfloat16, 8, "bhsd"),
+])
+def test_one_query_row(cuda_device, B, H, Sk, D, dtype, kv_heads, layout):
+    """Decoding: keys split over warps and cluster CTAs, ragged ends, shared K/V heads, LSE."""
+    gen = torch.Generator(device=cuda_device).manual_seed(Sk + D)
+
+    def make(heads, s):
+        shape = (B, s, heads, D) if layout == "bshd" else (B, heads, s, D)
+        t = torch.empty(shape, device=cuda_device).normal_(generator=gen).to(dtype)
+        return t.transpose(1, 2) if layout == "bshd" else t
+
+    q, k, v = make(H, 1), make(kv_heads, Sk), make(kv_heads, Sk)
+    k[:, :, Sk // 2] *= 4  # a maximum in the middle of a split
+    k, v = k.expand(-1, H, -1, -1), v.expand(-1, H, -1, -1)
+    o, lse = flash_attention_forward(q, k, v, return_lse=True)
+    s = (q.double() @ k.double().transpose(-1, -2)) / D ** 0.5
+    want = torch.softmax(s, -1) @ v.double()
+    # fp32 throughout, one rounding of the result (half an ulp of 8 significant bits in bf16, 11 in
+    # fp16: 2^-8 and 2^-11 of the value); sums of Sk terms of size <= 5 in fp32 stay within 1e-5
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert ((o.double() - want).abs() <= 1.01 * rel * want.abs() + 2e-5).all()
+    assert torch.allclose(lse.double(), torch.logsumexp(s, -1), atol=1e-4, rtol=1e-5)
+
+
+def test_one_query_row_causal_sees_key_zero_and_graph_replay(cuda_device):
+    q, k, v = (torch.randn(2, 3, s, 64, device=cuda_device, dtype=torch.bfloat16) for s in (1, 700, 700))
+    assert torch.equal(flash_attention_forward(q, k, v, causal=True), v[:, :, :1])
+    eager = flash_attention_forward(q, k, v)
+    out = torch.empty_like(q)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        flash_attention_forward(q, k, v, out=out)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
+
+
+@pytest.mark.parametrize("bad", ["batch_stride_0", "row_stride", "base"])
+def test_one_query_row_refuses_what_the_tiled_path_refuses(cuda_device, bad):
+    q = torch.randn(2, 3, 1, 64, device=cuda_device, dtype=torch.bfloat16)
+    k = torch.randn(2, 3, 64, 64, device=cuda_device, dtype=torch.bfloat16)
+    if bad == "batch_stride_0":
+        k = k[:1].expand(2, -1, -1, -1)
+    elif bad == "row_stride":
+        k = torch.randn(2, 3, 64, 68, device=cuda_device, dtype=torch.bfloat16)[..., :64]
+    else:
+        k = torch.randn(2 * 3 * 64 * 64 + 4, device=cuda_device, dtype=torch.bfloat16)[4:].view(2, 3, 64, 64)
+    with pytest.raises(RuntimeError):
+        flash_attention_forward(q, k, k)
