@@ -17,6 +17,7 @@ FO_F16, FO_BF16, FO_F32 = 0, 1, 2
 
 _lock = threading.Lock()
 _lib = None
+_raw_stream = None  # torch's accessor of the current raw stream, looked up on first use
 
 _c = ctypes
 _PTR = _c.c_void_p
@@ -139,17 +140,23 @@ def dtype_code(dtype) -> int:
 
 
 def current_stream_ptr(device) -> int:
-    """Raw cudaStream_t of torch's current stream on `device` (the cheap accessor when this torch
-    has it: constructing a torch.cuda.Stream object costs a few microseconds per call)."""
-    import torch
+    """Raw cudaStream_t of torch's current stream on `device` (a torch.device or an index; the
+    cheap accessor when this torch has it: constructing a torch.cuda.Stream object costs a few
+    microseconds per call)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
 
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if raw is not None:
-        index = device.index if isinstance(device, torch.device) else int(device)
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda i: torch.cuda.current_stream(i).cuda_stream)
+    if type(device) is not int:
+        index = device.index
         if index is None:
+            import torch
+
             index = torch.cuda.current_device()
-        return raw(index)
-    return torch.cuda.current_stream(device).cuda_stream
+        device = index
+    return _raw_stream(device)
 
 
 def device_status(device_index: int, reset: bool = False) -> int:

@@ -46,13 +46,15 @@ inline cudaError_t ensure_dynamic_smem(int bytes, int device) {
   return e;
 }
 
-// RAII: make `device` current for the scope, restore the previous one afterwards.
+// RAII: make `device` current for the scope, restore the previous one afterwards.  The device is set
+// even when it already is the thread's device: a thread that has made no runtime call yet (an
+// autograd worker) has no context bound, and the driver call that encodes tensor maps needs one.
 struct DeviceGuard {
   int prev = -1;
   bool ok = false;
   explicit DeviceGuard(int device) {
     if (cudaGetDevice(&prev) != cudaSuccess) return;
-    if (prev != device && cudaSetDevice(device) != cudaSuccess) return;
+    if (cudaSetDevice(device) != cudaSuccess) return;
     ok = true;
     want = device;
   }

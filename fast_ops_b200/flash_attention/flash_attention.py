@@ -21,16 +21,21 @@ from torch.autograd import Function
 from .. import _lib
 
 
-def _strides3(t: Tensor):
-    return (ctypes.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
+_I64x3 = ctypes.c_int64 * 3
+_CODES = {torch.float16: _lib.FO_F16, torch.bfloat16: _lib.FO_BF16}
 
 
-def _prepare_bias(bias: Optional[Tensor], Q: Tensor, N: int):
+def _strides3(t: Tensor, bshd: bool = False):
+    """(batch, head, row) strides of a (B, H, S, D) tensor, or of a (B, S, H, D) one."""
+    s = t.stride()
+    return _I64x3(s[0], s[2], s[1]) if bshd else _I64x3(s[0], s[1], s[2])
+
+
+def _prepare_bias(bias: Optional[Tensor], Q: Tensor, B: int, H: int, M: int, N: int):
     """Checks a bias the way the reference does (flash_attention_triton.py:752-769) and returns
     (tensor kept alive, pointer, stride array, dtype code) for the C ABI."""
     if bias is None:
         return None, None, None, _lib.FO_F32
-    B, H, M, _ = Q.shape
     if bias.dtype not in (Q.dtype, torch.float32):
         raise RuntimeError(f"bias must be float32 or have Q's dtype, got {bias.dtype}")
     if not bias.is_cuda or bias.device != Q.device:
@@ -39,12 +44,14 @@ def _prepare_bias(bias: Optional[Tensor], Q: Tensor, N: int):
         raise RuntimeError("bias must be 4-D, broadcastable to (B, H, M, N)")
     if bias.stride(-1) != 1:
         bias = bias.contiguous()
-    if tuple(bias.shape[2:]) not in ((1, N), (M, N)):
+    shape, st = bias.shape, bias.stride()
+    if shape[3] != N or shape[2] not in (1, M):
         raise RuntimeError("Last 2 dimensions of bias must be (1, seqlen_k) or (seqlen_q, seqlen_k)")
-    if bias.shape[0] not in (1, B) or bias.shape[1] not in (1, H):
+    if shape[0] not in (1, B) or shape[1] not in (1, H):
         raise RuntimeError("bias batch and head dimensions must be 1 or match Q")
-    bias = bias.expand(B, H, M, N)
-    return bias, bias.data_ptr(), _strides3(bias), _lib.dtype_code(bias.dtype)
+    # the strides of bias.expand(B, H, M, N): 0 where one row, head or batch serves several
+    strides = _I64x3(*(0 if shape[i] != full else st[i] for i, full in enumerate((B, H, M))))
+    return bias, bias.data_ptr(), strides, _lib.FO_F32 if bias.dtype == torch.float32 else _CODES[bias.dtype]
 
 
 def next_dropout_rng(device: torch.device, count: int) -> Tuple[int, int]:
@@ -101,22 +108,36 @@ def flash_attention_forward(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool = F
     Q's dtype, plus LSE (B, H, M) fp32 when `return_lse`.  `out`, if given, receives O: shape
     (B, H, M, D), Q's dtype and device, last dimension contiguous (any layout otherwise).
     """
+    return _forward(Q, K, V, False, causal, softmax_scale, return_lse, out, bias, dropout_p, rng)
+
+
+def _forward(Q: Tensor, K: Tensor, V: Tensor, bshd: bool, causal: bool, softmax_scale: Optional[float],
+             return_lse: bool, out: Optional[Tensor], bias: Optional[Tensor], dropout_p: float,
+             rng: Optional[Tuple[int, int]]):
+    """The forward call on (B, H, S, D) tensors or, with `bshd`, on (B, S, H, D) ones (only the
+    strides handed to the kernel differ, nothing is transposed); O has the layout of Q's dimensions."""
     if not (isinstance(Q, Tensor) and isinstance(K, Tensor) and isinstance(V, Tensor)):
         raise RuntimeError("Q, K, V must be tensors")
     if Q.dim() != 4 or K.dim() != 4 or V.dim() != 4:
-        raise RuntimeError("Q, K, V must be 4-D (B, H, S, D)")
+        raise RuntimeError("Q, K, V must be 4-D")
     if not Q.is_cuda:
         raise RuntimeError("fast_ops_b200 attention needs CUDA tensors (there is no CPU path)")
-    if K.device != Q.device or V.device != Q.device:
+    dev = Q.get_device()
+    if not K.is_cuda or not V.is_cuda or K.get_device() != dev or V.get_device() != dev:
         raise RuntimeError("Q, K, V must be on the same device")
-    if Q.dtype not in (torch.float16, torch.bfloat16):
+    code = _CODES.get(Q.dtype)
+    if code is None:
         raise RuntimeError(f"inputs must be float16 or bfloat16, got {Q.dtype}")
     if K.dtype != Q.dtype or V.dtype != Q.dtype:
         raise RuntimeError("Q, K, V must have the same dtype")
-    B, H, M, D = Q.shape
-    if K.shape[0] != B or K.shape[1] != H or K.shape[3] != D or V.shape != K.shape:
+    if bshd:
+        B, M, H, D = Q.shape
+        KB, N, KH, KD = K.shape
+    else:
+        B, H, M, D = Q.shape
+        KB, KH, N, KD = K.shape
+    if KB != B or KH != H or KD != D or V.shape != K.shape:
         raise RuntimeError(f"shape mismatch: Q {tuple(Q.shape)}, K {tuple(K.shape)}, V {tuple(V.shape)}")
-    N = K.shape[2]
     if D > 128 or D % 8 != 0:
         raise RuntimeError(f"head_dim must be a multiple of 8 and <= 128, got {D}")
     for name, t in (("Q", Q), ("K", K), ("V", V)):
@@ -125,32 +146,31 @@ def flash_attention_forward(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool = F
     scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
 
     if out is None:
-        O = torch.empty((B, H, M, D), dtype=Q.dtype, device=Q.device)
+        O = torch.empty_like(Q, memory_format=torch.contiguous_format)
     else:
-        if out.shape != (B, H, M, D) or out.dtype != Q.dtype or out.device != Q.device or out.stride(3) != 1:
+        if out.shape != Q.shape or out.dtype != Q.dtype or out.device != Q.device or out.stride(3) != 1:
             raise RuntimeError("out must be (B, H, M, D) with Q's dtype and device and a contiguous last dimension")
         O = out
-    lse = torch.empty((B, H, M), dtype=torch.float32, device=Q.device) if return_lse else None
+    lse = Q.new_empty((B, H, M), dtype=torch.float32) if return_lse else None
     lib = _lib.load()
     if bias is None and dropout_p == 0.0:
         rc = lib.fo_flash_attn_fwd(
             Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse.data_ptr() if return_lse else None,
-            B, H, M, N, D, _strides3(Q), _strides3(K), _strides3(V), _strides3(O),
-            _lib.dtype_code(Q.dtype), int(bool(causal)), scale, Q.device.index,
-            _lib.current_stream_ptr(Q.device))
+            B, H, M, N, D, _strides3(Q, bshd), _strides3(K, bshd), _strides3(V, bshd), _strides3(O, bshd),
+            code, int(bool(causal)), scale, dev, _lib.current_stream_ptr(dev))
     else:
         if not 0.0 <= dropout_p < 1.0:
             raise RuntimeError(f"dropout_p must be in [0, 1), got {dropout_p}")
         if dropout_p > 0.0 and rng is None:
             raise RuntimeError("dropout needs rng=(seed, offset); see next_dropout_rng")
         seed, offset = rng if rng is not None else (0, 0)
-        bias_t, bias_ptr, bias_strides, bias_code = _prepare_bias(bias, Q, N)
+        bias_t, bias_ptr, bias_strides, bias_code = _prepare_bias(bias, Q, B, H, M, N)
         rc = lib.fo_flash_attn_fwd_ex(
             Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse.data_ptr() if return_lse else None,
-            B, H, M, N, D, _strides3(Q), _strides3(K), _strides3(V), _strides3(O),
-            _lib.dtype_code(Q.dtype), int(bool(causal)), scale,
+            B, H, M, N, D, _strides3(Q, bshd), _strides3(K, bshd), _strides3(V, bshd), _strides3(O, bshd),
+            code, int(bool(causal)), scale,
             bias_ptr, bias_strides, bias_code, float(dropout_p), seed & (2**64 - 1), offset & (2**64 - 1),
-            Q.device.index, _lib.current_stream_ptr(Q.device))
+            dev, _lib.current_stream_ptr(dev))
     _lib.check(rc)
     return (O, lse) if return_lse else O
 
@@ -170,21 +190,35 @@ def flash_attention_backward(dO: Tensor, Q: Tensor, K: Tensor, V: Tensor, O: Ten
     returns with `return_lse=True`.  Semantics of the reference's complete backward
     (fast_ops/flash_attention/flash_attention_triton.py:832-958).
     """
+    return _backward(dO, Q, K, V, O, LSE, False, causal, softmax_scale, bias, dropout_p, rng)
+
+
+def _backward(dO: Tensor, Q: Tensor, K: Tensor, V: Tensor, O: Tensor, LSE: Tensor, bshd: bool, causal: bool,
+              softmax_scale: Optional[float], bias: Optional[Tensor], dropout_p: float,
+              rng: Optional[Tuple[int, int]]) -> Tuple[Tensor, Tensor, Tensor]:
+    """The backward call on (B, H, S, D) tensors or, with `bshd`, on (B, S, H, D) ones."""
+    dtype, dev = Q.dtype, Q.get_device()
     for name, t in (("dO", dO), ("Q", Q), ("K", K), ("V", V), ("O", O)):
-        if not t.is_cuda or t.dim() != 4 or t.dtype != Q.dtype or t.device != Q.device:
+        if not t.is_cuda or t.dim() != 4 or t.dtype != dtype or t.get_device() != dev:
             raise RuntimeError(f"{name} must be a 4-D CUDA tensor with Q's dtype and device")
         if t.stride(3) != 1:
             raise RuntimeError(f"{name}: the last dimension must be contiguous")
-    if Q.dtype not in (torch.float16, torch.bfloat16):
-        raise RuntimeError(f"inputs must be float16 or bfloat16, got {Q.dtype}")
-    B, H, M, D = Q.shape
-    N = K.shape[2]
-    if dO.shape != Q.shape or O.shape != Q.shape or V.shape != K.shape or K.shape[:2] != (B, H) or K.shape[3] != D:
+    code = _CODES.get(dtype)
+    if code is None:
+        raise RuntimeError(f"inputs must be float16 or bfloat16, got {dtype}")
+    if bshd:
+        B, M, H, D = Q.shape
+        KB, N, KH, KD = K.shape
+    else:
+        B, H, M, D = Q.shape
+        KB, KH, N, KD = K.shape
+    if dO.shape != Q.shape or O.shape != Q.shape or V.shape != K.shape or KB != B or KH != H or KD != D:
         raise RuntimeError("shape mismatch between dO, Q, K, V, O")
     if LSE.shape != (B, H, M) or LSE.dtype != torch.float32 or not LSE.is_contiguous() or LSE.device != Q.device:
         raise RuntimeError("LSE must be a contiguous (B, H, M) float32 tensor on Q's device")
     scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
-    if K.stride(1) == 0 or V.stride(1) == 0:
+    head = 2 if bshd else 1
+    if K.stride(head) == 0 or V.stride(head) == 0:
         # multi-query K/V expanded over the heads: the kernel writes one dK, dV per query head
         # (autograd sums them through the expand), so it needs per-head storage to read from too
         K, V = K.contiguous(), V.contiguous()
@@ -192,29 +226,32 @@ def flash_attention_backward(dO: Tensor, Q: Tensor, K: Tensor, V: Tensor, O: Ten
     for t in (dQ, dK, dV):
         if t.stride(3) != 1:
             raise RuntimeError("gradient layout: the last dimension must be contiguous")
-    dq_accum = torch.empty((B, H, M, D), dtype=torch.float32, device=Q.device)
-    delta = torch.empty((B, H, M), dtype=torch.float32, device=Q.device)
+    # one scratch block: the fp32 dQ accumulator (B, H, M, D), then rowsum(O o dO) (B, H, M)
+    rows = B * H * M
+    scratch = Q.new_empty((rows * (D + 1),), dtype=torch.float32)
+    dq_accum = scratch.data_ptr()
+    delta = dq_accum + 4 * rows * D
     lib = _lib.load()
     if bias is None and dropout_p == 0.0:
         rc = lib.fo_flash_attn_bwd(
             Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), dO.data_ptr(), LSE.data_ptr(),
-            dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(), dq_accum.data_ptr(), delta.data_ptr(),
-            B, H, M, N, D, _strides3(Q), _strides3(K), _strides3(V), _strides3(O), _strides3(dO),
-            _strides3(dQ), _strides3(dK), _strides3(dV),
-            _lib.dtype_code(Q.dtype), int(bool(causal)), scale, Q.device.index, _lib.current_stream_ptr(Q.device))
+            dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(), dq_accum, delta,
+            B, H, M, N, D, _strides3(Q, bshd), _strides3(K, bshd), _strides3(V, bshd), _strides3(O, bshd),
+            _strides3(dO, bshd), _strides3(dQ, bshd), _strides3(dK, bshd), _strides3(dV, bshd),
+            code, int(bool(causal)), scale, dev, _lib.current_stream_ptr(dev))
     else:
         if dropout_p > 0.0 and rng is None:
             raise RuntimeError("dropout needs the forward's rng=(seed, offset)")
         seed, offset = rng if rng is not None else (0, 0)
-        bias_t, bias_ptr, bias_strides, bias_code = _prepare_bias(bias, Q, N)
+        bias_t, bias_ptr, bias_strides, bias_code = _prepare_bias(bias, Q, B, H, M, N)
         rc = lib.fo_flash_attn_bwd_ex(
             Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), dO.data_ptr(), LSE.data_ptr(),
-            dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(), dq_accum.data_ptr(), delta.data_ptr(),
-            B, H, M, N, D, _strides3(Q), _strides3(K), _strides3(V), _strides3(O), _strides3(dO),
-            _strides3(dQ), _strides3(dK), _strides3(dV),
-            _lib.dtype_code(Q.dtype), int(bool(causal)), scale,
+            dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(), dq_accum, delta,
+            B, H, M, N, D, _strides3(Q, bshd), _strides3(K, bshd), _strides3(V, bshd), _strides3(O, bshd),
+            _strides3(dO, bshd), _strides3(dQ, bshd), _strides3(dK, bshd), _strides3(dV, bshd),
+            code, int(bool(causal)), scale,
             bias_ptr, bias_strides, bias_code, float(dropout_p), seed & (2**64 - 1), offset & (2**64 - 1),
-            Q.device.index, _lib.current_stream_ptr(Q.device))
+            dev, _lib.current_stream_ptr(dev))
     _lib.check(rc)
     return dQ, dK, dV
 
@@ -223,38 +260,38 @@ class _AttentionFunction(Function):
     """Forward + backward with the keyword arguments carried as non-tensor inputs.
 
     `rng` is the (seed, offset) pair of the dropout mask, or None to draw it from the device's
-    generator when `dropout_p` > 0; with `bshd_out` O is allocated as a (B, S, H, D) block and
-    returned as its (B, H, S, D) view, so that the caller's transpose back is contiguous."""
+    generator when `dropout_p` > 0; with `bshd` the tensors are (B, S, H, D).  The LSE is an output
+    only if the caller wants it: an output that nobody uses would get a gradient of zeros allocated
+    and filled on every backward."""
 
     @staticmethod
     def forward(ctx, Q: Tensor, K: Tensor, V: Tensor, causal: bool, softmax_scale: Optional[float],
                 bias: Optional[Tensor], dropout_p: float, rng: Optional[Tuple[int, int]] = None,
-                bshd_out: bool = False):
+                bshd: bool = False, return_lse: bool = False):
         if rng is None and dropout_p > 0.0:
             # one index per attention probability (flash_attention_triton.py:780)
-            rng = next_dropout_rng(Q.device, Q.shape[0] * Q.shape[1] * Q.shape[2] * K.shape[2])
-        out = None
-        if bshd_out:
-            B, H, M, D = Q.shape
-            out = torch.empty((B, M, H, D), dtype=Q.dtype, device=Q.device).transpose(1, 2)
-        O, lse = flash_attention_forward(Q, K, V, causal=causal, softmax_scale=softmax_scale, return_lse=True,
-                                         bias=bias, dropout_p=dropout_p, rng=rng, out=out)
+            rng = next_dropout_rng(Q.device, Q.shape[0] * Q.shape[1] * Q.shape[2] * K.shape[1 if bshd else 2])
+        O, lse = _forward(Q, K, V, bshd, causal, softmax_scale, True, None, bias, dropout_p, rng)
         ctx.save_for_backward(Q, K, V, O, lse, bias)
-        ctx.causal, ctx.softmax_scale, ctx.dropout_p, ctx.rng = causal, softmax_scale, dropout_p, rng
+        ctx.causal, ctx.softmax_scale, ctx.dropout_p, ctx.rng, ctx.bshd = causal, softmax_scale, dropout_p, rng, bshd
+        if not return_lse:
+            return O
+        ctx.set_materialize_grads(False)
         ctx.mark_non_differentiable(lse)
         return O, lse
 
     @staticmethod
-    def backward(ctx, dO: Tensor, _dlse):
+    def backward(ctx, dO: Optional[Tensor], _dlse=None):
+        none = (None,) * 7
+        if dO is None:
+            return (None, None, None) + none
         Q, K, V, O, lse, bias = ctx.saved_tensors
         if bias is not None and ctx.needs_input_grad[5]:
             raise RuntimeError("attention bias gradient is not supported")  # flash_attention_triton.py:854
         if dO.stride(3) != 1:
             dO = dO.contiguous()
-        dQ, dK, dV = flash_attention_backward(dO, Q, K, V, O, lse, causal=ctx.causal,
-                                              softmax_scale=ctx.softmax_scale, bias=bias,
-                                              dropout_p=ctx.dropout_p, rng=ctx.rng)
-        return dQ, dK, dV, None, None, None, None, None, None
+        return _backward(dO, Q, K, V, O, lse, ctx.bshd, ctx.causal, ctx.softmax_scale, bias, ctx.dropout_p,
+                         ctx.rng) + none
 
 
 class FlashAttentionFunction(Function):
@@ -263,7 +300,7 @@ class FlashAttentionFunction(Function):
 
     @staticmethod
     def forward(ctx, Q: Tensor, K: Tensor, V: Tensor) -> Tensor:
-        O, lse = flash_attention_forward(Q, K, V, return_lse=True)
+        O, lse = _forward(Q, K, V, False, False, None, True, None, None, 0.0, None)
         ctx.save_for_backward(Q, K, V, O, lse)
         return O
 
@@ -272,7 +309,7 @@ class FlashAttentionFunction(Function):
         Q, K, V, O, lse = ctx.saved_tensors
         if dO.stride(3) != 1:
             dO = dO.contiguous()
-        return flash_attention_backward(dO, Q, K, V, O, lse)
+        return _backward(dO, Q, K, V, O, lse, False, False, None, None, 0.0, None)
 
 
 def multi_head_attention(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool = False,
@@ -294,8 +331,8 @@ def multi_head_attention(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool = Fals
     if not causal and softmax_scale is None and not return_lse and bias is None and dropout_p == 0.0:
         return FlashAttentionFunction.apply(Q, K, V)
     if torch.is_grad_enabled() and (Q.requires_grad or K.requires_grad or V.requires_grad):
-        O, lse = _AttentionFunction.apply(Q, K, V, bool(causal), softmax_scale, bias, float(dropout_p))
-        return (O, lse) if return_lse else O
+        return _AttentionFunction.apply(Q, K, V, bool(causal), softmax_scale, bias, float(dropout_p), None, False,
+                                        return_lse)
     rng = None
     if dropout_p > 0.0:
         rng = next_dropout_rng(Q.device, Q.shape[0] * Q.shape[1] * Q.shape[2] * K.shape[2])

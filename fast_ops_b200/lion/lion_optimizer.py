@@ -106,7 +106,8 @@ class _TensorList:
 
     def __init__(self, key, params: List[Tensor], grads: List[Tensor], moms: List[Tensor]):
         n = len(params)
-        self.key = key
+        _, self.device_index, p_dtype, m_dtype = key
+        self.p_code, self.m_code = _lib.dtype_code(p_dtype), _lib.dtype_code(m_dtype)
         self.n = n
         self.params = (ctypes.c_void_p * n)(*[t.data_ptr() for t in params])
         self.grads = (ctypes.c_void_p * n)(*[t.data_ptr() for t in grads])
@@ -191,12 +192,9 @@ class Lion(Optimizer):
             weight_decay = float(group["weight_decay"])
             beta1, beta2 = (float(b) for b in group["betas"])
             for tl in cached[1]:
-                _, device_index, p_dtype, m_dtype = tl.key
                 _lib.check(lib.fo_lion_multi_tensor_step(
-                    tl.params, tl.grads, tl.moms, tl.numels, tl.n,
-                    _lib.dtype_code(p_dtype), _lib.dtype_code(p_dtype), _lib.dtype_code(m_dtype),
-                    lr, beta1, beta2, weight_decay, device_index,
-                    _lib.current_stream_ptr(torch.device("cuda", device_index))))
+                    tl.params, tl.grads, tl.moms, tl.numels, tl.n, tl.p_code, tl.p_code, tl.m_code,
+                    lr, beta1, beta2, weight_decay, tl.device_index, _lib.current_stream_ptr(tl.device_index)))
 
     def load_state_dict(self, state_dict) -> None:
         """As torch.optim.Optimizer.load_state_dict; in process_group mode the loaded momentum

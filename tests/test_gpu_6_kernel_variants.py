@@ -88,3 +88,25 @@ def test_one_query_row_refuses_what_the_tiled_path_refuses(cuda_device, bad):
         k = torch.randn(2 * 3 * 64 * 64 + 4, device=cuda_device, dtype=torch.bfloat16)[4:].view(2, 3, 64, 64)
     with pytest.raises(RuntimeError):
         flash_attention_forward(q, k, k)
+
+
+def test_a_thread_without_a_cuda_context_can_call(cuda_device):
+    """The tensor maps are encoded by a driver call that needs a context on the calling thread."""
+    import threading
+
+    q = torch.randn(1, 2, 136, 64, device=cuda_device, dtype=torch.bfloat16)
+    out, result = torch.empty_like(q), []
+    want = flash_attention_forward(q, q, q)
+    torch.cuda.synchronize()
+
+    def call():
+        try:
+            result.append(flash_attention_forward(q, q, q, out=out, softmax_scale=0.125))
+        except RuntimeError as e:
+            result.append(e)
+
+    t = threading.Thread(target=call)
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert result[0] is out and torch.equal(out, want)
