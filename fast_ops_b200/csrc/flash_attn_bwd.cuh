@@ -172,7 +172,9 @@ __device__ __forceinline__ void load_bias_rows32(const AttnExtras& ex, const uin
 }
 
 // grid = (key tiles, B*H); block = BwdConfig<D, kExt>::kThreads.
-template <int D, bool kBf16, int kExt>
+// kMma is the head_dim that the matmuls compute, D the width of the tiles: the zero columns between
+// them are left out of the K Q^T and V dO^T steps and of the width of dV, dK and dQ.
+template <int D, bool kBf16, int kExt, int kMma = D>
 __global__ void __launch_bounds__(BwdConfig<D, kExt>::kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -566,12 +568,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (warp == kCW + 4) {
       // ================================ MMA issuer ================================
       constexpr uint32_t idesc_s = make_idesc(kBf16, kBlockN, kBlockM, 0, 0);  // S^T, dP^T: both K-major
-      constexpr uint32_t idesc_a = make_idesc(kBf16, kBlockN, D, 0, 1);        // dV, dK: A from tensor memory, B N-major
-      constexpr uint32_t idesc_q = make_idesc(kBf16, kBlockM, D, 1, 1);        // dQ: A M-major, B N-major
+      constexpr uint32_t idesc_a = make_idesc(kBf16, kBlockN, kMma, 0, 1);     // dV, dK: A from tensor memory, B N-major
+      constexpr uint32_t idesc_q = make_idesc(kBf16, kBlockM, kMma, 1, 1);     // dQ: A M-major, B N-major
       constexpr uint32_t kBoxStep = kBoxBytes >> 4;
       // 16 queries per step; a thread's 16-bit results sit in the first half of its kCols columns
-      constexpr int kStepsPerPart = Cfg::kCols / 16;
-      auto part_col = [](int kk) -> uint32_t { return (kk / kStepsPerPart) * Cfg::kCols + (kk % kStepsPerPart) * 8; };
+      // Four steps go out per election: one election per matmul step made the whole kernel 1.5 to 2 %
+      // slower (B2 H32 S4096 D128 757 against 748 us), a branch per step 10 %.
+      // (kCols = 64: columns 0-31 and 64-95; kCols = 32: 0-15, 32-47, 64-79, 96-111)
+      constexpr int kA1 = 8, kA2 = Cfg::kCols == 64 ? 16 : 32, kA3 = kA2 + 8;
       const uint32_t q_k = desc_lo(smem_u32(sQ), 16), do_k = desc_lo(smem_u32(sDO), 16);
       const uint32_t k_k = desc_lo(smem_u32(sK), 16), v_k = desc_lo(smem_u32(sV), 16);
       const uint32_t q_n = desc_lo(smem_u32(sQ), kBoxBytes), do_n = desc_lo(smem_u32(sDO), kBoxBytes);
@@ -581,34 +585,34 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint32_t tS = tmem_base + Cfg::kColS, tDP = tmem_base + Cfg::kColDP, tDQ = tmem_base + Cfg::kColDQ;
       constexpr int kSlotMask = Cfg::kSlots - 1, kSlotShift = Cfg::kSlots - 1;  // slot of tile t, and its phase (t >> shift) & 1
 
+      auto issue_head_dim = [&](uint32_t d, uint32_t a, uint32_t b) {  // d = A B^T over the kMma columns
+#pragma unroll
+        for (int x = 0; x < kMma / 64; ++x)  // a 64-column box is four 16-column slices, 32 bytes apart
+          umma_ss4_elect<2, 2>(d, a + x * kBoxStep, b + x * kBoxStep, idesc_s, x > 0 ? 1u : 0u);
+#pragma unroll
+        for (int kk = kMma / 64 * 4; kk < kMma / 16; ++kk)
+          umma_ss_lo_elect(d, a + (kk >> 2) * kBoxStep + (kk & 3) * 2, b + (kk >> 2) * kBoxStep + (kk & 3) * 2, idesc_s, 1u);
+      };
       auto issue_st = [&](int t) {  // S^T = K Q^T of query tile t  (K = head_dim)
         mbar_wait(bar_q_full + (t & 1), (t >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
         tcgen05_fence_after_sync();
         const uint32_t qs = q_k + (t & 1) * (kTileBytes >> 4);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBoxStep + (kk & 3) * 2;
-          umma_ss_lo_elect(tS, k_k + off, qs + off, idesc_s, kk > 0 ? 1u : 0u);
-        }
+        issue_head_dim(tS, k_k, qs);
         tcgen05_commit_elect(bar_s_full);
       };
       auto issue_dpt = [&](int t) {  // dP^T = V dO^T of query tile t
         mbar_wait(bar_do_full + (t & kSlotMask), (t >> kSlotShift) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
         tcgen05_fence_after_sync();
         const uint32_t dos = do_k + (t & kSlotMask) * (kTileBytes >> 4);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBoxStep + (kk & 3) * 2;
-          umma_ss_lo_elect(tDP, v_k + off, dos + off, idesc_s, kk > 0 ? 1u : 0u);
-        }
+        issue_head_dim(tDP, v_k, dos);
         tcgen05_commit_elect(bar_dp_full);
       };
       auto issue_dq = [&](int t) {  // dQ = dS K  (K = 16 keys per step)
         const uint32_t ds = ds_m + (t & kSlotMask) * (Cfg::kDSBytes >> 4);
         const uint32_t d = tDQ + (kSepDQ ? (t & 1) * 64 : 0);
 #pragma unroll
-        for (int kk = 0; kk < kBlockN / 16; ++kk)
-          umma_ss_lo_elect(d, ds + kk * 128, k_n + kk * 128, idesc_q, kk > 0 ? 1u : 0u);
+        for (int x = 0; x < kBlockN / 64; ++x)
+          umma_ss4_elect<128, 128>(d, ds + x * 512, k_n + x * 512, idesc_q, x > 0 ? 1u : 0u);
         tcgen05_commit_elect(bar_dq_full + Cfg::par(t));
       };
       mbar_wait(bar_kv, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
@@ -623,8 +627,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         bwd_trace(prm, 2, it, 1);
         const uint32_t don = do_n + (it & kSlotMask) * (kTileBytes >> 4);
 #pragma unroll
-        for (int kk = 0; kk < kBlockM / 16; ++kk)  // dV += P^T dO
-          umma_ts_lo_elect(tDV, tS + part_col(kk), don + kk * 128, idesc_a, (it > 0 || kk > 0) ? 1u : 0u);
+        for (int x = 0; x < 2; ++x)  // dV += P^T dO
+          umma_ts4_elect<kA1, kA2, kA3, 128>(tDV, tS + x * 64, don + x * 512, idesc_a, (it > 0 || x > 0) ? 1u : 0u);
         tcgen05_commit_elect(bar_do_empty + (it & kSlotMask));  // dO_i has no reader after this point
         if (it + 1 < n_iter) issue_st(it + 1);  // over P^T, behind the matmul that reads it
         mbar_wait(bar_ds_full + Cfg::par(it), Cfg::phase(it), cta_abort, dstat, FO_STATUS_TIMEOUT_SOFTMAX);
@@ -632,8 +636,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         bwd_trace(prm, 2, it, 2);
         const uint32_t qn = q_n + (it & 1) * (kTileBytes >> 4);
 #pragma unroll
-        for (int kk = 0; kk < kBlockM / 16; ++kk)  // dK += dS^T Q
-          umma_ts_lo_elect(tDK, tDP + part_col(kk), qn + kk * 128, idesc_a, (it > 0 || kk > 0) ? 1u : 0u);
+        for (int x = 0; x < 2; ++x)  // dK += dS^T Q
+          umma_ts4_elect<kA1, kA2, kA3, 128>(tDK, tDP + x * 64, qn + x * 512, idesc_a, (it > 0 || x > 0) ? 1u : 0u);
         tcgen05_commit_elect(bar_q_empty + (it & 1));  // this Q slot has no reader after this point
         if constexpr (kSepDQ) {
           if (it + 1 < n_iter) issue_dpt(it + 1);  // over dS^T, behind the matmul that reads it

@@ -375,6 +375,7 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
     CUtensorMap tkh, tvh;
     if (int rc = make_tensor_map(&tkh, k, dtype, B, Hkv, Sk, D, k_strides, "k", fo::kStepN)) return rc;
     if (int rc = make_tensor_map(&tvh, v, dtype, B, Hkv, Sk, D, v_strides, "v", fo::kStepN)) return rc;
+    if (D > 64 && D <= 96) return bf16 ? fo::launch_ws64s<128, true, 96>(tq, tkh, tvh, prm, s) : fo::launch_ws64s<128, false, 96>(tq, tkh, tvh, prm, s);
     if (Dk == 128) return bf16 ? fo::launch_ws64s<128, true>(tq, tkh, tvh, prm, s) : fo::launch_ws64s<128, false>(tq, tkh, tvh, prm, s);
     return bf16 ? fo::launch_ws64s<64, true>(tq, tkh, tvh, prm, s) : fo::launch_ws64s<64, false>(tq, tkh, tvh, prm, s);
   }
@@ -384,6 +385,8 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
     impl = AttnImpl::kWarpSpecialized64;
   }
   if (impl == AttnImpl::kWarpSpecialized64) {
+    if (mode == 0 && D > 64 && D <= 96)
+      return bf16 ? fo::launch_ws64<128, true, 0, 96>(tq, tk, tv, prm, s) : fo::launch_ws64<128, false, 0, 96>(tq, tk, tv, prm, s);
     FO_WS_MODE(launch_ws64, 0)
     FO_WS_MODE(launch_ws64, 1)
     FO_WS_MODE(launch_ws64, 2)

@@ -433,6 +433,64 @@ __device__ __forceinline__ void umma_ts_lo_elect(uint32_t d_tmem, uint32_t a_tme
       : "memory");
 }
 
+// Four K = 16 steps of one matmul in one asm block: one election for the four, the second to fourth
+// accumulating.  kA / kB are the steps between consecutive slices (descriptor units of 16 bytes for
+// a shared-memory operand, columns for a tensor-memory one).  How fast the issuing warp gets its
+// instructions out bounds the attention kernels: see the figures at the issuers.
+template <int kA, int kB>
+__device__ __forceinline__ void umma_ss4_elect(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, t, e;\n\t"
+      ".reg .b64 da0, db0, da1, db1, da2, db2, da3, db3;\n\t"
+      ".reg .b32 a1, b1, a2, b2, a3, b3;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 a1, %1, %6;\n\t add.u32 b1, %2, %7;\n\t"
+      "add.u32 a2, %1, %8;\n\t add.u32 b2, %2, %9;\n\t"
+      "add.u32 a3, %1, %10;\n\t add.u32 b3, %2, %11;\n\t"
+      "mov.b64 da0, {%1, %3};\n\t mov.b64 db0, {%2, %3};\n\t"
+      "mov.b64 da1, {a1, %3};\n\t mov.b64 db1, {b1, %3};\n\t"
+      "mov.b64 da2, {a2, %3};\n\t mov.b64 db2, {b2, %3};\n\t"
+      "mov.b64 da3, {a3, %3};\n\t mov.b64 db3, {b3, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da0, db0, %4, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da1, db1, %4, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da2, db2, %4, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da3, db3, %4, t;\n\t"
+      "}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate),
+        "n"(kA), "n"(kB), "n"(2 * kA), "n"(2 * kB), "n"(3 * kA), "n"(3 * kB)
+      : "memory");
+}
+
+template <int kA1, int kA2, int kA3, int kB>
+__device__ __forceinline__ void umma_ts4_elect(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, t, e;\n\t"
+      ".reg .b64 db0, db1, db2, db3;\n\t"
+      ".reg .b32 a1, b1, a2, b2, a3, b3;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 a1, %1, %6;\n\t add.u32 b1, %2, %9;\n\t"
+      "add.u32 a2, %1, %7;\n\t add.u32 b2, %2, %10;\n\t"
+      "add.u32 a3, %1, %8;\n\t add.u32 b3, %2, %11;\n\t"
+      "mov.b64 db0, {%2, %3};\n\t mov.b64 db1, {b1, %3};\n\t"
+      "mov.b64 db2, {b2, %3};\n\t mov.b64 db3, {b3, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db0, %4, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], db1, %4, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], db2, %4, t;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], db3, %4, t;\n\t"
+      "}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate),
+        "n"(kA1), "n"(kA2), "n"(kA3), "n"(kB), "n"(2 * kB), "n"(3 * kB)
+      : "memory");
+}
+
 __device__ __forceinline__ void tcgen05_commit_elect(uint64_t* bar) {
   asm volatile(
       "{\n\t"

@@ -110,3 +110,22 @@ def test_a_thread_without_a_cuda_context_can_call(cuda_device):
     t.join()
     torch.cuda.synchronize()
     assert result[0] is out and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("D", [72, 80, 96, 104])
+@pytest.mark.parametrize("impl", ["ws64", "ws64s"])
+def test_head_dims_around_the_96_column_kernels(cuda_device, D, impl):
+    """72 to 96 run matmuls of width 96, 104 those of width 128: forward and backward against the oracle."""
+    import fast_ops_b200._lib as L
+
+    B, H, Sq, Sk = 1, 2, 260, 330
+    gen = torch.Generator().manual_seed(D)
+    q, dout = (torch.randn(B, H, Sq, D, generator=gen).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, H, Sk, D, generator=gen).bfloat16() for _ in range(2))
+    L.attn_configure(impl=impl)
+    try:
+        got, _, same, _ = run_case(cuda_device, q, k, v, dout, False, None, 0.0, None)
+    finally:
+        L.attn_configure(impl="auto")
+    out, _, dq, dk, dv = oracle.attention_ex(q, k, v, causal=False, dout=dout)
+    check(got, same, (out, dq, dk, dv), f"D={D} {impl}")
