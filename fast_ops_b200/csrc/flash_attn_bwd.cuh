@@ -90,7 +90,7 @@ struct BwdConfig {
   // head_dim 64 with dropout or a matrix bias: sixteen compute warps (four threads per key row, 32
   // query columns each) instead of eight.  Hashing and fetching bias values are long chains per
   // thread, and eight warps do not cover their latency: B2 H16 S2048 D64 with both 472 us with
-  // sixteen warps, 702 with eight (391 and not timed once vector and matrix bias were compiled apart).  Without them eight warps are the faster form (B8 H12 S1024 D64
+  // sixteen warps, 702 with eight (391 with sixteen since vector and matrix bias are compiled apart).  Without them eight warps are the faster form (B8 H12 S1024 D64
   // causal 81 against 84 us), and at head_dim 128 the registers do not reach.
   static constexpr bool kWide = D == 64 && (kExt & (kBwdDropout | kBwdMatBias)) != 0;
   static constexpr int kComputeWarps = kWide ? 16 : 8;
