@@ -85,6 +85,10 @@ __device__ __forceinline__ void load_bias32(const AttnExtras& ex, const uint8_t*
   }
 }
 
+// kExt of the 64-key kernel for a bias, the variants compiled: a bias that is the same for every query row
+// ("vector"), dropout, a bias with a row stride ("matrix").
+constexpr int kFwdVecBias = 1, kFwdDropout = 2, kFwdMatBias = 4;
+
 struct AttnParams {
   void* o;
   float* lse;  // may be null
@@ -158,6 +162,12 @@ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t tile_smem, int kk) {
 // N (head_dim) is the contiguous direction, consecutive 64-wide column blocks are kBoxBytes apart.
 __device__ __forceinline__ uint64_t nmajor_desc(uint32_t tile_smem, int kk) {
   return smem_desc(tile_smem + kk * 2048, kBoxBytes, 1024);
+}
+
+template <bool kBf16>
+__device__ __forceinline__ float2 unpack2(uint32_t w) {
+  if constexpr (kBf16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  else return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
 
 template <bool kBf16>

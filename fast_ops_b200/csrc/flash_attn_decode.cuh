@@ -45,12 +45,6 @@ struct DecodeParams {
 constexpr int kDecodeThreads = 256;
 constexpr int kDecodeWarps = kDecodeThreads / 32;
 
-template <bool kBf16>
-__device__ __forceinline__ float2 unpack2(uint32_t w) {
-  if constexpr (kBf16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-  else return __half22float2(*reinterpret_cast<const __half2*>(&w));
-}
-
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"

@@ -15,6 +15,7 @@
 #include "flash_attn_ws.cuh"
 #include "flash_attn_ws64.cuh"
 #include "flash_attn_ws64p.cuh"
+#include "flash_attn_ws64r.cuh"
 #include "flash_attn_ws64s.cuh"
 #include "fo_host.h"
 #include "fo_tma.h"
@@ -388,9 +389,16 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
     if (mode == 0 && D > 64 && D <= 96)
       return bf16 ? fo::launch_ws64<128, true, 0, 96>(tq, tk, tv, prm, s) : fo::launch_ws64<128, false, 0, 96>(tq, tk, tv, prm, s);
     FO_WS_MODE(launch_ws64, 0)
-    FO_WS_MODE(launch_ws64, 1)
     FO_WS_MODE(launch_ws64, 2)
-    FO_WS_MODE(launch_ws64, 3)
+    // with a bias: the kernel that takes the keys in descending order, vector and matrix compiled apart
+    const int drop = mode & fo::kFwdDropout;
+    {
+      const int mode = (prm.ex.bias_stride_q == 0 ? fo::kFwdVecBias : fo::kFwdMatBias) | drop;
+      FO_WS_MODE(launch_ws64r, 1)
+      FO_WS_MODE(launch_ws64r, 3)
+      FO_WS_MODE(launch_ws64r, 4)
+      FO_WS_MODE(launch_ws64r, 6)
+    }
   }
   if (impl != AttnImpl::kSimple || mode != 0) {
     FO_WS_MODE(launch_ws, 0)
