@@ -1,0 +1,62 @@
+// The order in which a warp that issues matmuls takes the entries of a ring of K and V tiles.
+// Plain C++, so that the same code runs in the kernel and in a model of the ring's barriers on the CPU.
+//
+// Entry 2 j is the K tile of key tile j in the CTA's order, entry 2 j + 1 its V tile; entry e is the
+// (e / kStages)-th use of slot e % kStages, and its load completes phase e / kStages of the slot's
+// "full" barrier.  A slot is loaded again once both issuing warps have released it.
+//
+// A barrier is waited on by the parity of a phase: the wait for phase f returns as soon as the
+// barrier is not in phase f - 1 + 2 n, so a warp that has not seen phase f - 1 end may be let
+// through one load early, and loads do not complete in the order they were requested in.  Hence the
+// rule that this walk keeps: a warp waits for every entry, in order within a slot, also for those it
+// only passes over.
+#pragma once
+
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define FO_RING_FN __device__ __forceinline__
+#else
+#define FO_RING_FN inline
+#endif
+
+namespace fo {
+
+// The walk of a warp whose query tile takes T >= 2 steps of half a key tile each, of key tiles j0 to
+// n - 1 of the ring (those before j0 belong to the CTA's other query tile).
+//   ops.wait(slot, parity)      blocks until that phase of the slot's "full" barrier is complete
+//   ops.ready(slot, parity)     the same without blocking
+//   ops.release(slot)           this warp's readers of the slot have all been issued
+//   ops.first_scores(slot)      issues the scores of steps 0 and 1, whose K tile is in `slot`
+//   ops.step(t, v_slot, k_slot) issues P V of step t and the scores of step t + 2 if there is one
+template <int kStages, class Ops>
+FO_RING_FN void walk_kv_ring(int j0, int n, int T, const Ops& ops) {
+  auto slot = [](int e) { return e % kStages; };
+  auto parity = [](int e) { return static_cast<uint32_t>((e / kStages) & 1); };
+  for (int e = 0; e < 2 * j0; ++e) {
+    ops.wait(slot(e), parity(e));
+    ops.release(slot(e));
+  }
+  ops.wait(slot(2 * j0), parity(2 * j0));
+  ops.first_scores(slot(2 * j0));
+  ops.release(slot(2 * j0));
+  bool ready = false;  // looked at one step ahead, waited for only if that look failed
+  for (int t = 0; t < T; ++t) {
+    const int j = (t >> 1) + j0;
+    const int v = 2 * j + 1, k = v + 1;  // V of this step's key tile, K of the next
+    const bool k_next = j + 1 < n;
+    if ((t & 1) == 0 && !ready) {
+      ops.wait(slot(v), parity(v));
+      if (k_next) ops.wait(slot(k), parity(k));
+    }
+    ready = false;
+    ops.step(t, slot(v), slot(k));
+    if ((t & 1) == 1 || t + 1 == T) {
+      ops.release(slot(v));
+      if (k_next) ops.release(slot(k));
+      if (t + 1 < T) ready = ops.ready(slot(v + 2), parity(v + 2)) && (!(j + 2 < n) || ops.ready(slot(k + 2), parity(k + 2)));
+    }
+  }
+}
+
+}  // namespace fo

@@ -13,6 +13,7 @@
 // order in which the assembler places the exponentials around the turn-taking barriers changes).
 #pragma once
 
+#include "flash_attn_ring.h"
 #include "flash_attn_ws64.cuh"
 
 namespace fo {
@@ -545,66 +546,50 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
       };
 
-      mbar_wait(bar_q_full, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
-      // key tiles of the ring that only tile 1 reads (0 or 1): released unread
-      const int j0 = s ? 0 : skip0 >> 1;
-      for (int i = 0; i < 2 * j0; ++i) tcgen05_commit_elect(bar_kv_empty + i);
-      const int st0 = 2 * j0;  // ring slot of this tile's first K (the ring has at least 4)
-      mbar_wait(bar_kv_full + st0, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
-      tcgen05_fence_after_sync();
-      // prologue: the first two steps, both on that K tile
-      issue_s(0, st0);
-      tcgen05_commit_elect(bar_s_full + 2 * s);
-      if (T_s > 1) {
-        issue_s(1, st0);
+      auto wait_kv = [&](int slot, uint32_t parity) {
+        mbar_wait(bar_kv_full + slot, parity, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
+      };
+      auto kv_ready = [&](int slot, uint32_t parity) { return mbar_test_wait(bar_kv_full + slot, parity); };
+      auto release_kv = [&](int slot) { tcgen05_commit_elect(bar_kv_empty + slot); };
+      auto first_scores = [&](int slot) {
+        tcgen05_fence_after_sync();
+        issue_s(0, slot);
+        tcgen05_commit_elect(bar_s_full + 2 * s);
+        issue_s(1, slot);
         tcgen05_commit_elect(bar_s_full + 2 * s + 1);
-      }
-      tcgen05_commit_elect(bar_kv_empty + st0);
-      // Barriers are polled (without blocking) one iteration ahead and waited on only if the
-      // poll failed.
-      bool p_ready = false, kv_ready = false;
-      const int t_end = T_s;
-      for (int t = 0; t < t_end; ++t) {
-        const int j = (t >> 1) + j0, u = t & 1;
-        const int iv = 2 * j + 1;  // ring index of V_j; K_{j+1} is iv + 1
-        const int st_v = iv % kStages;
-        const int st_k = (iv + 1) % kStages;
-        const bool k_next = j + 1 < n1;  // K_{j+1} exists
-        if (u == 0 && !kv_ready) {
-          mbar_wait(bar_kv_full + st_v, (iv / kStages) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
-          if (k_next) mbar_wait(bar_kv_full + st_k, ((iv + 1) / kStages) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
-        }
+      };
+      // P is polled (without blocking) one step ahead and waited for only if the poll failed.
+      bool p_ready = false;
+      auto step = [&](int t, int v_slot, int k_slot) {
+        const int u = t & 1;
         if (s == 0) trace_event(prm, 2, t, 0);
-        kv_ready = false;
-        if (t < T_s) {
-          if (!p_ready)
-            mbar_wait(bar_p_full + 2 * s + u, (t >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_SOFTMAX);
-          tcgen05_fence_after_sync();
-          if (s == 0) trace_event(prm, 2, t, 1);
-          issue_pv(u, st_v, t > 0);
-          tcgen05_commit_elect(bar_o_full + s);
-          if (t + 1 == T_s) tcgen05_commit_elect(bar_o_done + s);
-          if (s == 0) trace_event(prm, 2, t, 2);
-          // step t + 2 goes into the buffer that P(s, t) is being read from; the tensor core runs
-          // one thread's instructions in order, so the read comes first
-          if (t + 2 < T_s) {
-            issue_s(u, st_k);
-            tcgen05_commit_elect(bar_s_full + 2 * s + u);
-          }
-          if (s == 0) trace_event(prm, 2, t, 3);
-          p_ready = (t + 1 < T_s) && mbar_test_wait(bar_p_full + 2 * s + (u ^ 1), ((t + 1) >> 1) & 1);
+        if (!p_ready)
+          mbar_wait(bar_p_full + 2 * s + u, (t >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_SOFTMAX);
+        tcgen05_fence_after_sync();
+        if (s == 0) trace_event(prm, 2, t, 1);
+        issue_pv(u, v_slot, t > 0);
+        tcgen05_commit_elect(bar_o_full + s);
+        if (t + 1 == T_s) tcgen05_commit_elect(bar_o_done + s);
+        if (s == 0) trace_event(prm, 2, t, 2);
+        // step t + 2 goes into the buffer that P(s, t) is being read from; the tensor core runs
+        // one thread's instructions in order, so the read comes first
+        if (t + 2 < T_s) {
+          issue_s(u, k_slot);
+          tcgen05_commit_elect(bar_s_full + 2 * s + u);
         }
-        if (u == 1 || t + 1 == t_end) {
-          // this warp's readers of V_j (and of K_{j+1}) have all been issued
-          tcgen05_commit_elect(bar_kv_empty + st_v);
-          if (k_next) tcgen05_commit_elect(bar_kv_empty + st_k);
-          if (t + 1 < t_end) {
-            const int iv2 = iv + 2;
-            kv_ready = mbar_test_wait(bar_kv_full + iv2 % kStages, (iv2 / kStages) & 1) &&
-                       (!(j + 2 < n1) || mbar_test_wait(bar_kv_full + (iv2 + 1) % kStages, ((iv2 + 1) / kStages) & 1));
-          }
-        }
-      }
+        if (s == 0) trace_event(prm, 2, t, 3);
+        p_ready = (t + 1 < T_s) && mbar_test_wait(bar_p_full + 2 * s + (u ^ 1), ((t + 1) >> 1) & 1);
+      };
+      mbar_wait(bar_q_full, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
+      struct {
+        decltype(wait_kv) wait;
+        decltype(kv_ready) ready;
+        decltype(release_kv) release;
+        decltype(first_scores) first_scores;
+        decltype(step) step;
+      } const ops{wait_kv, kv_ready, release_kv, first_scores, step};
+      // the ring's first key tile is read by tile 1 alone if tile 0 joins later
+      walk_kv_ring<kStages>(s ? 0 : skip0 >> 1, n1, T_s, ops);
     } else if (warp == 13) {
       // ================================ TMA producer ================================
       const bool issuer = lane == 0;
