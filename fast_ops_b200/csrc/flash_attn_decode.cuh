@@ -42,9 +42,6 @@ struct DecodeParams {
   const int* device_status;
 };
 
-constexpr int kDecodeThreads = 256;
-constexpr int kDecodeWarps = kDecodeThreads / 32;
-
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -53,8 +50,12 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 }
 
 // grid = (cluster size * head groups, B); a head group is kHeads heads (1 when K and V are per head).
-template <int D, bool kBf16, int kHeads>
-__global__ void __launch_bounds__(kDecodeThreads, kHeads == 1 ? 2 : 1)
+// Blocks of kWarps warps that one SM holds: 16 warps of the per-head form, 8 of the shared-head form.
+template <int kHeads, int kWarps>
+constexpr int kDecodePerSm = (kHeads == 1 ? 16 : 8) / kWarps;
+
+template <int D, bool kBf16, int kHeads, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, kDecodePerSm<kHeads, kWarps>)
 attn_decode_kernel(const DecodeParams prm) {
   namespace cg = cooperative_groups;
   constexpr int kLanes = D / 8;        // lanes per key row
@@ -72,8 +73,8 @@ attn_decode_kernel(const DecodeParams prm) {
   const bool d_ok = d0 < prm.d_real;  // d_real is a multiple of 8; missing columns are zeros
 
   // One row per (warp or CTA) partial result: D values of the unnormalised output, maximum, sum.
-  __shared__ __align__(16) float s_part[kDecodeWarps][kHeads][D];
-  __shared__ float s_ml[kDecodeWarps][kHeads][2];
+  __shared__ __align__(16) float s_part[kWarps][kHeads][D];
+  __shared__ float s_ml[kWarps][kHeads][2];
   __shared__ __align__(16) float s_cta[kHeads][D];        // this CTA's partial, read by the cluster's rank 0
   __shared__ float s_cta_ml[kHeads][2];
 
@@ -123,7 +124,7 @@ attn_decode_kernel(const DecodeParams prm) {
   uint4 kw[kBatch], vw[kBatch];
   int base = begin + warp * kStep;
   if (base < end) load_rows(kw, kp, prm.k_stride_s, base);
-  for (; base < end; base += kDecodeWarps * kStep) {
+  for (; base < end; base += kWarps * kStep) {
     load_rows(vw, vp, prm.v_stride_s, base);
     float s[kHeads];
 #pragma unroll
@@ -153,7 +154,7 @@ attn_decode_kernel(const DecodeParams prm) {
       s[r] = (base + group * kBatch + own < end) ? t[0] : -INFINITY;
     }
     // K of the next step: its registers are free now
-    if (base + kDecodeWarps * kStep < end) load_rows(kw, kp, prm.k_stride_s, base + kDecodeWarps * kStep);
+    if (base + kWarps * kStep < end) load_rows(kw, kp, prm.k_stride_s, base + kWarps * kStep);
     float p[kHeads];
 #pragma unroll
     for (int r = 0; r < kHeads; ++r) {
@@ -207,15 +208,15 @@ attn_decode_kernel(const DecodeParams prm) {
   }
   __syncthreads();
   // ---- CTA ----
-  for (int x = tid; x < kHeads * D; x += kDecodeThreads) {
+  for (int x = tid; x < kHeads * D; x += kWarps * 32) {
     const int r = x / D, d = x % D;
     float mx = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kDecodeWarps; ++w) mx = fmaxf(mx, s_ml[w][r][0]);
+    for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, s_ml[w][r][0]);
     const float m_use = mx == -INFINITY ? 0.f : mx;
     float a = 0.f, sum = 0.f;
 #pragma unroll
-    for (int w = 0; w < kDecodeWarps; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       const float f = fast_exp2(s_ml[w][r][0] - m_use);
       a = fmaf(f, s_part[w][r][d], a);
       sum = fmaf(f, s_ml[w][r][1], sum);
@@ -230,7 +231,7 @@ attn_decode_kernel(const DecodeParams prm) {
   // ---- cluster: rank 0 reads every CTA's partial through distributed shared memory ----
   // (nothing is stored while the device's status word says that an earlier launch gave up)
   if (rank == 0 && *reinterpret_cast<const volatile int*>(prm.device_status) == 0) {
-    for (int x = tid; x < kHeads * (D / 2); x += kDecodeThreads) {
+    for (int x = tid; x < kHeads * (D / 2); x += kWarps * 32) {
       const int r = x / (D / 2), d = (x % (D / 2)) * 2;
       const int h = h0 + r;
       if (h >= prm.H) continue;
@@ -258,7 +259,7 @@ attn_decode_kernel(const DecodeParams prm) {
 
 // CTAs of this kernel that can be resident together in clusters of 16 (asked once per device; the
 // largest cluster must find all its SMs inside one GPC, so the chip holds fewer of them).
-template <auto kKernel>
+template <auto kKernel, int kThreads>
 inline int resident_ctas_in_clusters_of_16(int device) {
   static std::atomic<int> known[64];  // CTAs + 1, 0 = not asked yet
   if (device < 0 || device >= 64) return 0;
@@ -267,7 +268,7 @@ inline int resident_ctas_in_clusters_of_16(int device) {
     int clusters = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(kDecodeThreads);
+    cfg.blockDim = dim3(kThreads);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 16;
@@ -286,33 +287,68 @@ inline int resident_ctas_in_clusters_of_16(int device) {
   return n - 1;
 }
 
-template <int D, bool kBf16, int kHeads>
-int launch_decode(const DecodeParams& base, int B, int num_sms, int device, cudaStream_t stream) {
-  constexpr auto kernel = attn_decode_kernel<D, kBf16, kHeads>;
+// How the keys are divided: heads per CTA, warps per CTA, CTAs per head (0: launch_decode decides).
+struct DecodeShape {
+  int heads, warps, split;
+};
+
+// Up to 1024 keys the work of a CTA is a few steps, and what counts is how many rounds of CTAs the chip
+// takes, not how many warps share a head.  The shape with the least cost = rounds * (steps of a warp + 4),
+// in steps of eight rows per lane group, a step of the four-head form counting 1.3; a later candidate (four
+// heads, fewer warps, more CTAs) has to be 5 % ahead.  The constants are a fit to measured times: over
+// 64 to 4096 heads, one to 1000 keys, head_dim 64 and 128, it is within 2 % of the best shape on average
+// and 15 % at most.  Against eight warps throughout (us, head_dim 128, keys per head): 640 heads, 300:
+// 32.2 -> 21.1; 384, 300: 17.4 -> 10.6; 4096, 300: 128 -> 105; 4096, 64: 59.5 -> 30.7; one K/V head
+// shared by 32 query heads, 64 keys: 5.4 -> 4.2.  Beyond 1024 keys the bandwidth evens the shapes out and
+// the rule of launch_decode is the better one (640 heads, 1500 keys: 93 by this rule, 89 by that one).
+inline DecodeShape decode_shape(int B, int H, int Sk, int D, bool shared_kv, int num_sms) {
+  if (Sk > 1024) return {shared_kv ? 4 : 1, 8, 0};
+  const int rows = D <= 64 ? 32 : 16;  // rows of a warp's step
+  DecodeShape best = {1, 8, 1};
+  double best_cost = 0;
+  for (int heads = 1; heads <= (shared_kv ? 4 : 1); heads += 3)
+    for (int warps = 8; warps >= 2; warps /= 2)
+      for (int split = 1; split <= 8 && (split == 1 || Sk / split >= 64); split *= 2) {
+        const int64_t ctas = static_cast<int64_t>((H + heads - 1) / heads) * B * split;
+        const int slots = num_sms * ((heads == 1 ? 16 : 8) / warps);
+        const int steps = (Sk + split * rows * warps - 1) / (split * rows * warps);
+        const double cost = static_cast<double>((ctas + slots - 1) / slots) * (steps * (heads == 1 ? 1.0 : 1.3) + 4);
+        if (best_cost == 0 || cost < 0.95 * best_cost) {
+          best_cost = cost;
+          best = {heads, warps, split};
+        }
+      }
+  return best;
+}
+
+// `split`: CTAs that share a head's keys, or 0: the power of two up to 16 that takes the fewest rounds of
+// resident CTAs (two per SM, one in the shared-head form) per unit of split, the smaller unless
+// the larger saves 15 % of that (each doubling costs a little: more partial results, shorter
+// CTAs), while a CTA keeps at least 128 keys.  Measured at splits 1 / 2 / 4 / 8 / 16 (us):
+// B4 H32 Sk4096 D128 57 / 43 / 46 / 52 / 79 (takes 2); B1 H8 Sk32768 D128 389 / 197 / 101 / 54 / 36
+// (16); B8 H40 Sk3000 D96 92 / 82 / 80 / 96 (4).
+template <int D, bool kBf16, int kHeads, int kWarps>
+int launch_decode(const DecodeParams& base, int B, int split, int num_sms, int device, cudaStream_t stream) {
+  constexpr auto kernel = attn_decode_kernel<D, kBf16, kHeads, kWarps>;
   const int64_t groups = static_cast<int64_t>((base.H + kHeads - 1) / kHeads) * B;
-  // How many CTAs share a head's keys: the power of two up to 16 that takes the fewest rounds of
-  // resident CTAs (two per SM, one in the shared-head form) per unit of split, the smaller unless
-  // the larger saves 15 % of that (each doubling costs a little: more partial results, shorter
-  // CTAs), while a CTA keeps at least 128 keys.  Measured at splits 1 / 2 / 4 / 8 / 16 (us):
-  // B4 H32 Sk4096 D128 57 / 43 / 46 / 52 / 79 (takes 2); B1 H8 Sk32768 D128 389 / 197 / 101 / 54 / 36
-  // (16); B32 H8 Sk512 D128 14 / 17 / 22 / 38 (1); B8 H40 Sk3000 D96 92 / 82 / 80 / 96 (4).
-  const int resident = num_sms * (kHeads == 1 ? 2 : 1);
-  int split = 1;
-  double best = 0;
-  for (int s = 1; s <= 16 && (s == 1 || base.Sk / s >= 128); s *= 2) {
-    const int slots = s == 16 ? resident_ctas_in_clusters_of_16<kernel>(device) : resident;
-    if (slots < s) break;
-    const double cost = static_cast<double>((groups * s + slots - 1) / slots) / s;
-    if (s == 1 || cost < 0.85 * best) {
-      best = cost;
-      split = s;
+  if (split == 0) {
+    const int resident = num_sms * kDecodePerSm<kHeads, kWarps>;
+    double best = 0;
+    for (int s = 1; s <= 16 && (s == 1 || base.Sk / s >= 128); s *= 2) {
+      const int slots = s == 16 ? resident_ctas_in_clusters_of_16<kernel, kWarps * 32>(device) : resident;
+      if (slots < s) break;
+      const double cost = static_cast<double>((groups * s + slots - 1) / slots) / s;
+      if (s == 1 || cost < 0.85 * best) {
+        best = cost;
+        split = s;
+      }
     }
   }
   DecodeParams prm = base;
   prm.chunk = ((base.Sk + split - 1) / split + 15) / 16 * 16;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(groups / B * split), B);
-  cfg.blockDim = dim3(kDecodeThreads);
+  cfg.blockDim = dim3(kWarps * 32);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

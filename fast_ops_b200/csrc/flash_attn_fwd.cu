@@ -243,17 +243,20 @@ static int decode(const void* q, const void* k, const void* v, void* o, float* l
   prm.scale_log2 = softmax_scale * 1.4426950408889634f;
   prm.device_status = status;
   const bool bf16 = dtype == FO_BF16;
-  // Heads that share K and V go four to a CTA, so that the shared tensors cross L2 a quarter as often.
-#define FO_DECODE(DK, HEADS)                                                                 \
-  return bf16 ? fo::launch_decode<DK, true, HEADS>(prm, B, num_sms, device, stream)          \
-              : fo::launch_decode<DK, false, HEADS>(prm, B, num_sms, device, stream)
-  if (D <= 64) {
-    if (kv_bcast) FO_DECODE(64, 4);
-    FO_DECODE(64, 1);
-  }
-  if (kv_bcast) FO_DECODE(128, 4);
-  FO_DECODE(128, 1);
+  // Heads that share K and V may go four to a CTA, so that the shared tensors cross L2 a quarter as often.
+  const fo::DecodeShape shape = fo::decode_shape(B, H, Sk, D, kv_bcast, num_sms);
+#define FO_DECODE(DK, HEADS, WARPS)                                                                                \
+  if ((DK == 64) == (D <= 64) && shape.heads == HEADS && shape.warps == WARPS)                                     \
+    return bf16 ? fo::launch_decode<DK, true, HEADS, WARPS>(prm, B, shape.split, num_sms, device, stream)          \
+                : fo::launch_decode<DK, false, HEADS, WARPS>(prm, B, shape.split, num_sms, device, stream);
+#define FO_DECODE_WARPS(DK, HEADS) FO_DECODE(DK, HEADS, 8) FO_DECODE(DK, HEADS, 4) FO_DECODE(DK, HEADS, 2)
+  FO_DECODE_WARPS(64, 1)
+  FO_DECODE_WARPS(64, 4)
+  FO_DECODE_WARPS(128, 1)
+  FO_DECODE_WARPS(128, 4)
+#undef FO_DECODE_WARPS
 #undef FO_DECODE
+  return fo::fail(FO_ERR_UNSUPPORTED, "no decoding kernel of this shape");
 }
 
 static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, float* lse,

@@ -63,6 +63,26 @@ def test_one_query_row(cuda_device, B, H, Sk, D, dtype, kv_heads, layout):
     assert torch.allclose(lse.double(), torch.logsumexp(s, -1), atol=1e-4, rtol=1e-5)
 
 
+@pytest.mark.parametrize("B,H,shared", [(1, 8, False), (1, 8, True), (4, 32, False), (4, 32, True), (32, 12, False),
+                                        (32, 12, True), (16, 40, False), (16, 40, True), (64, 33, True)])
+@pytest.mark.parametrize("Sk", [1, 17, 64, 129, 300, 513, 1000, 1024, 1025])
+@pytest.mark.parametrize("D", [40, 128])
+def test_one_query_row_shapes(cuda_device, B, H, shared, Sk, D):
+    """Few to many heads, few to many keys: one or four heads per CTA, two to eight warps, one to eight
+    CTAs per head.  Every shape against the same call in 64 bits."""
+    gen = torch.Generator(device=cuda_device).manual_seed(B + Sk)
+    q = torch.empty(B, H, 1, D, device=cuda_device).normal_(generator=gen).bfloat16()
+    k, v = (torch.empty(B, 1 if shared else H, Sk, D, device=cuda_device).normal_(generator=gen).bfloat16()
+            .expand(B, H, Sk, D) for _ in range(2))
+    o, lse = flash_attention_forward(q, k, v, return_lse=True)
+    for b in range(0, B, 5):  # a slice at a time: the 64-bit copies stay small
+        s = (q[b].double() @ k[b].double().transpose(-1, -2)) / D ** 0.5
+        want = torch.softmax(s, -1) @ v[b].double()
+        # one rounding to 8 significant bits; fp32 sums of Sk terms stay within 2e-5
+        assert ((o[b].double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 2e-5).all()
+        assert torch.allclose(lse[b].double(), torch.logsumexp(s, -1), atol=1e-4, rtol=1e-5)
+
+
 def test_one_query_row_causal_sees_key_zero_and_graph_replay(cuda_device):
     q, k, v = (torch.randn(2, 3, s, 64, device=cuda_device, dtype=torch.bfloat16) for s in (1, 700, 700))
     assert torch.equal(flash_attention_forward(q, k, v, causal=True), v[:, :, :1])
