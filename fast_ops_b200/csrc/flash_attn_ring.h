@@ -22,15 +22,15 @@
 
 namespace fo {
 
-// The walk of a warp whose query tile takes T >= 2 steps of half a key tile each, of key tiles j0 to
-// n - 1 of the ring (those before j0 belong to the CTA's other query tile).
+// The walk of a warp whose query tile takes the steps `first` (0 or 1) to T - 1, two per key tile, on the
+// key tiles j0 to n - 1 of the ring (those before j0 belong to the CTA's other query tile).
 //   ops.wait(slot, parity)      blocks until that phase of the slot's "full" barrier is complete
 //   ops.ready(slot, parity)     the same without blocking
 //   ops.release(slot)           this warp's readers of the slot have all been issued
-//   ops.first_scores(slot)      issues the scores of steps 0 and 1, whose K tile is in `slot`
+//   ops.scores(t, slot)         issues the scores of step t, one of the first two, whose K tile is in `slot`
 //   ops.step(t, v_slot, k_slot) issues P V of step t and the scores of step t + 2 if there is one
 template <int kStages, class Ops>
-FO_RING_FN void walk_kv_ring(int j0, int n, int T, const Ops& ops) {
+FO_RING_FN void walk_kv_ring(int j0, int n, int first, int T, const Ops& ops) {
   auto slot = [](int e) { return e % kStages; };
   auto parity = [](int e) { return static_cast<uint32_t>((e / kStages) & 1); };
   for (int e = 0; e < 2 * j0; ++e) {
@@ -38,14 +38,19 @@ FO_RING_FN void walk_kv_ring(int j0, int n, int T, const Ops& ops) {
     ops.release(slot(e));
   }
   ops.wait(slot(2 * j0), parity(2 * j0));
-  ops.first_scores(slot(2 * j0));
+  ops.scores(first, slot(2 * j0));
+  if (first == 0 && T > 1) ops.scores(1, slot(2 * j0));
   ops.release(slot(2 * j0));
+  if (first == 1 && T > 2) {
+    ops.wait(slot(2 * j0 + 2), parity(2 * j0 + 2));
+    ops.scores(2, slot(2 * j0 + 2));
+  }
   bool ready = false;  // looked at one step ahead, waited for only if that look failed
-  for (int t = 0; t < T; ++t) {
+  for (int t = first; t < T; ++t) {
     const int j = (t >> 1) + j0;
     const int v = 2 * j + 1, k = v + 1;  // V of this step's key tile, K of the next
     const bool k_next = j + 1 < n;
-    if ((t & 1) == 0 && !ready) {
+    if (((t & 1) == 0 || t == first) && !ready) {
       ops.wait(slot(v), parity(v));
       if (k_next) ops.wait(slot(k), parity(k));
     }

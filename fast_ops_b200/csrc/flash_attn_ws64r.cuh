@@ -79,14 +79,21 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // keys visible to query tile 0 / 1 of this pair, in 64-key steps (T) and 128-key tiles (n)
   const int vis0 = prm.causal ? min(prm.Sk, (2 * pair + 1) * kBlockM) : prm.Sk;
   const int vis1 = prm.causal ? min(prm.Sk, (2 * pair + 2) * kBlockM) : prm.Sk;
-  // Tile 0 of the pair joins `skip0` steps after tile 1, which has the tiles next to the diagonal.
   const int n0 = (vis0 + kBlockN - 1) / kBlockN;
   const int n1 = (vis1 + kBlockN - 1) / kBlockN;
-  const int T0 = 2 * n0;  // T1 >= T0 >= 1
-  const int T1 = 2 * n1;
-  const int skip0 = T1 - T0;
-  // first key of step t of a query tile with T steps
-  auto step_key = [](int t, int T) { return T * kStepN - kBlockN * ((t >> 1) + 1) + (t & 1) * kStepN; };
+  // The steps of a query tile are `first` to T - 1, two per key tile.  When the last key tile's upper
+  // half has no visible key, step 0 is left out (taken, with all its scores masked, it made 64 keys
+  // cost 38 us instead of 29 at B64 H12 D64, and 1088 keys 128 instead of 120 at B8 H16); its barrier
+  // phases are completed in the set-up, so that step numbers stand for buffers and phases as ever.
+  const int T0 = 2 * n0, T1 = 2 * n1;  // T1 >= T0 >= 2
+  const int first0 = (vis0 + kStepN - 1) / kStepN & 1, first1 = (vis1 + kStepN - 1) / kStepN & 1;
+  // Tile 0 of the pair joins `skip0` steps after tile 1, which has the tiles next to the diagonal.
+  const int skip0 = (T1 - first1) - (T0 - first0);
+  // First key of step t.  A key tile's lower half comes before its upper half (in the tile on the
+  // diagonal more rows see it), and behind it if step 0 is left out.
+  auto step_key = [](int t, int first, int T) {
+    return T * kStepN - kBlockN * ((t >> 1) + 1) + ((t & 1) ^ first) * kStepN;
+  };
 
   if (tid == 0) {
     *cta_abort = 0;
@@ -134,6 +141,17 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     (2 * pair + s) * kBlockM, h, b);
     for (int i = 0; i < first_fill; ++i) load_kv(i);
   }
+  // the phases of a step 0 that is left out
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    if (!(s ? first1 : first0)) continue;
+    if (warp >> 2 == s) mbar_arrive(bar_corr + 2 * s);
+    if (warp >> 2 == s || warp >> 2 == 2) mbar_arrive(bar_p_full + 2 * s);
+    if (warp == (s ? 14 : 12) && lane == 0) {
+      mbar_arrive(bar_s_full + 2 * s);
+      mbar_arrive(bar_o_full + s);
+    }
+  }
   if (warp == 12) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish_alloc_permit();
@@ -151,7 +169,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const int r = (warp & 3) * 32 + lane;
     const int q0 = (2 * pair + s) * kBlockM;
     const int row = q0 + r;
-    const int T_s = s ? T1 : T0;
+    const int T_s = s ? T1 : T0, first = s ? first1 : first0;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS_tile = tmem_base + Cfg::kColS0 + s * kBlockN + lane_base;
     float* alpha_slot = s_alpha + s * 256 + r;
@@ -179,7 +197,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       if (vec_bias) {
         bias_vec = static_cast<const uint8_t*>(prm.ex.bias) +
                    (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h) * (prm.ex.bias_f32 ? 4 : 2);
-        const int col = step_key(0, T_s) + r;
+        const int col = T_s * kStepN - kBlockN + r;
         bias_next = (col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
       }
     }
@@ -203,11 +221,11 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     uint32_t sr[2][32];  // scores of the current step (scaled and biased already when there is a bias)
 
-    // Stages the row-independent bias of the key tile that step `tn` (even) starts.
+    // Stages the row-independent bias of the key tile that step `tn` starts.
     auto stage_vec_bias = [&](int tn) {
       const int j = tn >> 1;
       sb[(j & 1) * 128 + r] = bias_next;
-      const int col = step_key(tn + 2, T_s) + r;  // of the key tile after this one (below 0: there is none)
+      const int col = T_s * kStepN - kBlockN * (j + 2) + r;  // of the key tile after this one (below 0: there is none)
       bias_next = (col >= 0 && col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
       // a buffer is rewritten two key tiles later, behind the barrier of the tile between
       named_barrier_sync(1 + s, 128);
@@ -223,7 +241,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     uint4 bias_raw[mat_bias ? 8 : 1];
     bool bias_held = false;
     auto fetch_mat_bias = [&](int tn) {
-      const int k0n = step_key(tn, T_s);
+      const int k0n = step_key(tn, first, T_s);
       bias_held = bias_row != nullptr && !prm.ex.bias_f32 && prm.ex.bias_vec && k0n + kStepN <= prm.Sk;
       if (bias_held) {
         const uint4* const p = reinterpret_cast<const uint4*>(bias_row + static_cast<int64_t>(k0n) * 2);
@@ -233,7 +251,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     };
     // Waits for those loads and applies bias and masks in place.
     auto prep_loads = [&](int tn) {
-      const int k0n = step_key(tn, T_s);
+      const int k0n = step_key(tn, first, T_s);
       const bool need_mask = (k0n + kStepN > prm.Sk) || (prm.causal && k0n + kStepN - 1 > q0);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -241,7 +259,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if ((warp & 3) == 0 && tn > 0) trace_event(prm, s, tn - 1, c == 0 ? 1 : 4);  // loads in
         if constexpr (kExt != 0) {
           if (vec_bias) {
-            const float4* bv = reinterpret_cast<const float4*>(sb + ((tn >> 1) & 1) * 128 + (tn & 1) * kStepN + c * 32);
+            const float4* bv = reinterpret_cast<const float4*>(sb + ((tn >> 1) & 1) * 128 + ((tn & 1) ^ first) * kStepN + c * 32);
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
               const float4 v4 = bv[i >> 2];  // the same address in every thread: a broadcast
@@ -300,16 +318,16 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       return fmaxf(fmaxf(mxa, mxb), fmaxf(mxc, mxd));
     };
 
-    // prologue: scores of step 0; their row maximum is the first reference maximum
+    // prologue: scores of the first step; their row maximum is the first reference maximum
     if constexpr (kExt != 0) {
-      if (vec_bias) stage_vec_bias(0);
+      if (vec_bias) stage_vec_bias(first);
     }
-    if constexpr (mat_bias) fetch_mat_bias(0);
-    mbar_wait(bar_s_full + 2 * s, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
+    if constexpr (mat_bias) fetch_mat_bias(first);
+    mbar_wait(bar_s_full + 2 * s + first, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
     tcgen05_fence_after_sync();
-    issue_load(0, 0);
-    issue_load(0, 1);
-    prep_loads(0);
+    issue_load(first, 0);
+    issue_load(first, 1);
+    prep_loads(first);
     m_run = row_max() * exp_scale;
 
     // The exponentials of a step do not wait for the step's own row maximum: they are taken
@@ -320,9 +338,9 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // exponentials taken again.  Each iteration then fetches step t + 1 (whose S the tensor core
     // finished meanwhile) behind the P stores, so that the latencies of the loads, of the P store
     // and of the barriers overlap instead of adding up.
-    for (int t = 0; t < T_s; ++t) {
+    for (int t = first; t < T_s; ++t) {
       const int u = t & 1;
-      const int k0 = step_key(t, T_s);
+      const int k0 = step_key(t, first, T_s);
       const uint32_t tS = tS_tile + u * kStepN;
       float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
       if (ping_pong) named_barrier_sync_dep(s ? kTurn1 : kTurn0, kTurnCount, neg_m);  // exponentials start after this
@@ -404,7 +422,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           if (vec_bias && u == 1) stage_vec_bias(t + 1);
           if constexpr (mat_bias) fetch_mat_bias(t + 1);
           if (mat_bias && bias_row != nullptr && t + 2 < T_s) {
-            const int c0 = step_key(t + 2, T_s);
+            const int c0 = step_key(t + 2, first, T_s);
             if (c0 < prm.Sk) prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0));
           }
         }
@@ -467,14 +485,15 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             (l_run > 0.f) ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
       }
     };
-    for (int g = 0; g < T1; ++g) {
+    for (int g = first1; g < T1; ++g) {
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int t = s ? g : g - skip0;
-        if (t < 0 || t >= (s ? T1 : T0)) continue;
+        const int first = s ? first1 : first0;
+        const int t = s ? g : g - first1 - skip0 + first0;
+        if (t < first) continue;
         mbar_wait(bar_corr + 2 * s + (t & 1), (t >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_SOFTMAX);
         const float alpha = s_alpha[s * 256 + (t & 1) * 128 + r];
-        if (t > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+        if (t > first && __any_sync(0xffffffffu, alpha != 1.f)) {
           // this step's P V is not issued before this warp arrives below; O is complete up to
           // the previous step once that step's P V has finished.  (The P V of step t - 2 is
           // known to have finished, since S of step t exists: the phase bit is unambiguous.)
@@ -511,7 +530,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // other, and nothing has to: each tile owns its S / P buffers and its O accumulator, and a
       // K/V ring slot is released by both warps (bar_kv_empty counts two arrivals).
       const int s = (warp == 14) ? 1 : 0;
-      const int T_s = s ? T1 : T0;
+      const int T_s = s ? T1 : T0, first = s ? first1 : first0;
       constexpr uint32_t idesc_qk = make_idesc(kBf16, kBlockM, kStepN, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc(kBf16, kBlockM, D, 0, 1);
       // Everything below is warp-uniform; only the tcgen05 instructions themselves are issued by
@@ -523,10 +542,10 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       constexpr uint32_t kBoxStep = kBoxBytes >> 4;
       const uint32_t tS_tile = tmem_base + Cfg::kColS0 + s * kBlockN;
       const uint32_t tO = tmem_base + Cfg::kColO0 + s * D;
-      // S(s, t) = Q_s K^T over keys [64 u, 64 u + 64) of the K tile in ring slot `stage`, u = t & 1:
-      // 64 rows of a K-major box are 64 * 128 bytes further on
+      // S(s, t) = Q_s K^T over the step's half of the K tile in ring slot `stage`, u = t & 1: 64 rows
+      // of a K-major box are 64 * 128 bytes further on
       auto issue_s = [&](int u, int stage) {
-        const uint32_t b_lo = kv_k_lo + stage * kStageStep + u * ((kStepN * 128) >> 4);
+        const uint32_t b_lo = kv_k_lo + stage * kStageStep + (u ^ first) * ((kStepN * 128) >> 4);
         const uint32_t tS = tS_tile + u * kStepN;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
@@ -535,10 +554,10 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           umma_ss_lo_elect(tS, q_lo + off, b_lo + off, idesc_qk, kk > 0 ? 1u : 0u);
         }
       };
-      // O_s (+)= P(s, t) V over key rows [64 u, 64 u + 64) of the V tile in ring slot `stage`
+      // O_s (+)= P(s, t) V over the step's half of the V tile in ring slot `stage`
       auto issue_pv = [&](int u, int stage, bool acc) {
         const uint32_t tP = tS_tile + u * kStepN;
-        const uint32_t b_lo = kv_v_lo + stage * kStageStep + u * (kStepN / 16) * 128;
+        const uint32_t b_lo = kv_v_lo + stage * kStageStep + (u ^ first) * (kStepN / 16) * 128;
 #pragma unroll
         for (int kk = 0; kk < kStepN / 16; ++kk) {
           // 16 key rows per slice: 2048 bytes of V, 8 packed columns of P
@@ -551,12 +570,10 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       };
       auto kv_ready = [&](int slot, uint32_t parity) { return mbar_test_wait(bar_kv_full + slot, parity); };
       auto release_kv = [&](int slot) { tcgen05_commit_elect(bar_kv_empty + slot); };
-      auto first_scores = [&](int slot) {
+      auto scores = [&](int t, int slot) {
         tcgen05_fence_after_sync();
-        issue_s(0, slot);
-        tcgen05_commit_elect(bar_s_full + 2 * s);
-        issue_s(1, slot);
-        tcgen05_commit_elect(bar_s_full + 2 * s + 1);
+        issue_s(t & 1, slot);
+        tcgen05_commit_elect(bar_s_full + 2 * s + (t & 1));
       };
       // P is polled (without blocking) one step ahead and waited for only if the poll failed.
       bool p_ready = false;
@@ -567,7 +584,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           mbar_wait(bar_p_full + 2 * s + u, (t >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_SOFTMAX);
         tcgen05_fence_after_sync();
         if (s == 0) trace_event(prm, 2, t, 1);
-        issue_pv(u, v_slot, t > 0);
+        issue_pv(u, v_slot, t > first);
         tcgen05_commit_elect(bar_o_full + s);
         if (t + 1 == T_s) tcgen05_commit_elect(bar_o_done + s);
         if (s == 0) trace_event(prm, 2, t, 2);
@@ -585,11 +602,11 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         decltype(wait_kv) wait;
         decltype(kv_ready) ready;
         decltype(release_kv) release;
-        decltype(first_scores) first_scores;
+        decltype(scores) scores;
         decltype(step) step;
-      } const ops{wait_kv, kv_ready, release_kv, first_scores, step};
-      // the ring's first key tile is read by tile 1 alone if tile 0 joins later
-      walk_kv_ring<kStages>(s ? 0 : skip0 >> 1, n1, T_s, ops);
+      } const ops{wait_kv, kv_ready, release_kv, scores, step};
+      // the ring's first key tile is read by tile 1 alone if tile 0 joins a whole key tile later
+      walk_kv_ring<kStages>(s ? 0 : n1 - n0, n1, first, T_s, ops);
     } else if (warp == 13) {
       // ================================ TMA producer ================================
       const bool issuer = lane == 0;

@@ -22,16 +22,16 @@ struct Ops {
   void wait(int slot, uint32_t parity) const { printf("w %d %u\n", slot, parity); }
   bool ready(int, uint32_t) const { return false; }
   void release(int slot) const { printf("r %d\n", slot); }
-  void first_scores(int slot) const { printf("k 0 %d\nk 1 %d\n", slot, slot); }
+  void scores(int t, int slot) const { printf("k %d %d\n", t, slot); }
   void step(int t, int v_slot, int k_slot) const {
     printf("v %d %d\n", t, v_slot);
     if (t + 2 < T) printf("k %d %d\n", t + 2, k_slot);
   }
 };
 int main(int, char** a) {
-  const int stages = atoi(a[1]), j0 = atoi(a[2]), n = atoi(a[3]), T = atoi(a[4]);
-  if (stages == 4) fo::walk_kv_ring<4>(j0, n, T, Ops{T});
-  else fo::walk_kv_ring<6>(j0, n, T, Ops{T});
+  const int stages = atoi(a[1]), j0 = atoi(a[2]), n = atoi(a[3]), first = atoi(a[4]), T = atoi(a[5]);
+  if (stages == 4) fo::walk_kv_ring<4>(j0, n, first, T, Ops{T});
+  else fo::walk_kv_ring<6>(j0, n, first, T, Ops{T});
 }
 """
 
@@ -44,8 +44,12 @@ def recorder(tmp_path_factory):
         f.write(RECORDER)
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, src, "-o", exe], check=True)
 
-    def record(stages, j0, n, T):
-        out = subprocess.run([exe, str(stages), str(j0), str(n), str(T)], check=True, capture_output=True, text=True).stdout
+    def record(stages, n, halves):
+        """The walk of a query tile that sees `halves` half key tiles, in a ring of n key tiles."""
+        first, T = halves % 2, (halves + 1) // 2 * 2
+        j0 = n - T // 2
+        args = [stages, j0, n, first, T]
+        out = subprocess.run([exe, *map(str, args)], check=True, capture_output=True, text=True).stdout
         ops = []
         for line in out.splitlines():
             kind, *num = line.split()
@@ -113,17 +117,22 @@ def run(stages, entries, warps, rng, order):
 
 @pytest.mark.parametrize("stages", [4, 6])
 @pytest.mark.parametrize("order", ["random", "reversed"])
-@pytest.mark.parametrize("n0,n1", [(1, 1), (1, 2), (2, 2), (2, 3), (3, 3), (3, 4), (4, 5), (6, 7), (9, 9), (9, 10)])
-def test_every_read_finds_its_entry(recorder, stages, order, n0, n1):
-    """Query tile 0 sees n0 key tiles, tile 1 n1 (one more under a causal mask); the ring holds n1."""
-    warps = [recorder(stages, n1 - n0, n1, 2 * n0), recorder(stages, 0, n1, 2 * n1)]
+@pytest.mark.parametrize("seen0,seen1", [(1, 1), (2, 2), (2, 3), (2, 4), (3, 3), (4, 4), (4, 5), (4, 6), (5, 5), (6, 7),
+                                         (6, 8), (8, 10), (11, 11), (12, 14), (17, 17), (18, 20), (19, 19)])
+def test_every_read_finds_its_entry(recorder, stages, order, seen0, seen1):
+    """Query tile 0 sees seen0 half key tiles, tile 1 seen1 (up to two more under a causal mask)."""
+    n1 = (seen1 + 1) // 2
+    warps = [recorder(stages, n1, seen) for seen in (seen0, seen1)]
+    for warp, seen in zip(warps, (seen0, seen1)):
+        assert sum(op[0] == "read" for op in warp) == 2 * seen  # K and V of every step
+        assert sum(op[0] == "release" for op in warp) == 2 * n1
     for seed in range(60):
         run(stages, 2 * n1, warps, random.Random(seed), order)
 
 
 def test_the_model_sees_a_wait_that_is_missing(recorder):
     """Passing over the first key tile without waiting for it lets a warp take entry 4 for loaded."""
-    warps = [recorder(4, 1, 3, 4), recorder(4, 0, 3, 6)]
+    warps = [recorder(4, 3, seen) for seen in (4, 6)]
     assert warps[0][:4] == [("wait", 0, 0), ("release", 0), ("wait", 1, 0), ("release", 1)]
     del warps[0][2], warps[0][0]
     with pytest.raises(AssertionError, match="reads entry"):
