@@ -38,8 +38,10 @@ __device__ __forceinline__ uint32_t dropout_hash(uint32_t idx, uint32_t seed) {
 }
 
 // out[i] = log2(e) * bias[col0 + i] for the 32 columns col0.. of one bias row (`rowp` points at
-// column 0 of the row, or is null for a row past the end); columns >= Sk give 0.
-template <bool kBf16>
+// column 0 of the row, or is null for a row past the end); columns >= Sk give 0.  kType: the bias's type
+// where the kernel is compiled for it.
+constexpr int kBiasAny = 0, kBias16 = 1, kBias32 = 2;
+template <bool kBf16, int kType = kBiasAny>
 __device__ __forceinline__ void load_bias32(const AttnExtras& ex, const uint8_t* rowp, int col0, int Sk,
                                             float (&out)[32]) {
   constexpr float kLog2e = 1.4426950408889634f;
@@ -49,7 +51,7 @@ __device__ __forceinline__ void load_bias32(const AttnExtras& ex, const uint8_t*
     return;
   }
   const bool full = ex.bias_vec && (col0 + 32 <= Sk);
-  if (ex.bias_f32) {
+  if (kType == kBiasAny ? ex.bias_f32 != 0 : kType == kBias32) {
     const float* p = reinterpret_cast<const float*>(rowp) + col0;
     if (full) {
 #pragma unroll
@@ -86,8 +88,8 @@ __device__ __forceinline__ void load_bias32(const AttnExtras& ex, const uint8_t*
 }
 
 // kExt of the 64-key kernel for a bias, the variants compiled: a bias that is the same for every query row
-// ("vector"), dropout, a bias with a row stride ("matrix").
-constexpr int kFwdVecBias = 1, kFwdDropout = 2, kFwdMatBias = 4;
+// ("vector"), dropout, a 16-bit or an fp32 bias with a row stride ("matrix").
+constexpr int kFwdVecBias = 1, kFwdDropout = 2, kFwdMatBias = 4, kFwdMatBias32 = 8;
 
 struct AttnParams {
   void* o;

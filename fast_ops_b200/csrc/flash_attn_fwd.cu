@@ -396,11 +396,14 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
     // with a bias: the kernel that takes the keys in descending order, vector and matrix compiled apart
     const int drop = mode & fo::kFwdDropout;
     {
-      const int mode = (prm.ex.bias_stride_q == 0 ? fo::kFwdVecBias : fo::kFwdMatBias) | drop;
+      const int form = prm.ex.bias_stride_q == 0 ? fo::kFwdVecBias : prm.ex.bias_f32 ? fo::kFwdMatBias32 : fo::kFwdMatBias;
+      const int mode = form | drop;
       FO_WS_MODE(launch_ws64r, 1)
       FO_WS_MODE(launch_ws64r, 3)
       FO_WS_MODE(launch_ws64r, 4)
       FO_WS_MODE(launch_ws64r, 6)
+      FO_WS_MODE(launch_ws64r, 8)
+      FO_WS_MODE(launch_ws64r, 10)
     }
   }
   if (impl != AttnImpl::kSimple || mode != 0) {

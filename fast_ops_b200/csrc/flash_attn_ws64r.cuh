@@ -18,7 +18,7 @@
 
 namespace fo {
 
-// kExt: kFwdVecBias or kFwdMatBias, with or without kFwdDropout.
+// kExt: kFwdVecBias, kFwdMatBias or kFwdMatBias32, with or without kFwdDropout.
 template <int D, bool kBf16, int kExt>
 __global__ void __launch_bounds__(512, 1)
 attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -174,8 +174,8 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t tS_tile = tmem_base + Cfg::kColS0 + s * kBlockN + lane_base;
     float* alpha_slot = s_alpha + s * 256 + r;
     float m_run = -INFINITY, l_run = 0.f;
-    constexpr bool vec_bias = (kExt & kFwdVecBias) != 0, mat_bias = (kExt & kFwdMatBias) != 0;
-    constexpr bool has_bias = vec_bias || mat_bias;
+    constexpr bool vec_bias = (kExt & kFwdVecBias) != 0, mat_bias16 = (kExt & kFwdMatBias) != 0;
+    constexpr bool mat_bias = mat_bias16 || (kExt & kFwdMatBias32) != 0;
     constexpr bool has_drop = (kExt & kFwdDropout) != 0;
     const uint8_t* bias_row = nullptr;
     uint32_t drop_row = 0;
@@ -188,7 +188,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                  static_cast<uint32_t>(row) * static_cast<uint32_t>(prm.Sk);
     }
     // with a bias the scores are scaled when the bias is added, not in the exponent
-    const float exp_scale = has_bias ? 1.f : prm.scale_log2;
+    const float exp_scale = 1.f;
     // a row-independent bias goes through shared memory, fetched one 128-key tile ahead
     const uint8_t* bias_vec = nullptr;
     float* sb = s_bias + s * 256;
@@ -238,15 +238,15 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // A 16-bit matrix bias whose rows are 16-byte aligned is fetched into registers ahead of the
     // step that adds it (every thread reads its own row: 128 bytes per step), other forms when they
     // are added.
-    uint4 bias_raw[mat_bias ? 8 : 1];
+    uint4 bias_raw[mat_bias16 ? 8 : 1];
     bool bias_held = false;
     auto fetch_mat_bias = [&](int tn) {
       const int k0n = step_key(tn, first, T_s);
-      bias_held = bias_row != nullptr && !prm.ex.bias_f32 && prm.ex.bias_vec && k0n + kStepN <= prm.Sk;
+      bias_held = bias_row != nullptr && prm.ex.bias_vec && k0n + kStepN <= prm.Sk;
       if (bias_held) {
         const uint4* const p = reinterpret_cast<const uint4*>(bias_row + static_cast<int64_t>(k0n) * 2);
 #pragma unroll
-        for (int i = 0; i < (mat_bias ? 8 : 1); ++i) bias_raw[i] = __ldg(p + i);
+        for (int i = 0; i < (mat_bias16 ? 8 : 1); ++i) bias_raw[i] = __ldg(p + i);
       }
     };
     // Waits for those loads and applies bias and masks in place.
@@ -271,11 +271,11 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           }
           if constexpr (mat_bias) {
             float bb[32];
-            if (bias_held) {
+            if (mat_bias16 && bias_held) {
               constexpr float kLog2e = 1.4426950408889634f;
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                const uint4 v = bias_raw[mat_bias ? c * 4 + i : 0];
+                const uint4 v = bias_raw[mat_bias16 ? c * 4 + i : 0];
                 const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int y = 0; y < 4; ++y) {
@@ -285,7 +285,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 }
               }
             } else {
-              load_bias32<kBf16>(prm.ex, bias_row, k0n + c * 32, prm.Sk, bb);
+              load_bias32<kBf16, mat_bias16 ? kBias16 : kBias32>(prm.ex, bias_row, k0n + c * 32, prm.Sk, bb);
             }
 #pragma unroll
             for (int i = 0; i < 32; ++i)
@@ -322,7 +322,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if constexpr (kExt != 0) {
       if (vec_bias) stage_vec_bias(first);
     }
-    if constexpr (mat_bias) fetch_mat_bias(first);
+    if constexpr (mat_bias16) fetch_mat_bias(first);
     mbar_wait(bar_s_full + 2 * s + first, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
     tcgen05_fence_after_sync();
     issue_load(first, 0);
@@ -420,7 +420,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // of step t is in pr.
         if constexpr (kExt != 0) {
           if (vec_bias && u == 1) stage_vec_bias(t + 1);
-          if constexpr (mat_bias) fetch_mat_bias(t + 1);
+          if constexpr (mat_bias16) fetch_mat_bias(t + 1);
           if (mat_bias && bias_row != nullptr && t + 2 < T_s) {
             const int c0 = step_key(t + 2, first, T_s);
             if (c0 < prm.Sk) prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0));
