@@ -128,11 +128,15 @@ __device__ __forceinline__ float load_bias1(const AttnExtras& ex, const uint8_t*
 }
 
 // L2 prefetch of the `ncols` bias elements of a row starting at column col0 (row pointer non-null,
-// columns clamped to Sk by the caller).
-__device__ __forceinline__ void prefetch_bias(const AttnExtras& ex, const uint8_t* rowp, int col0, int ncols) {
+// columns clamped to Sk by the caller).  One line per 128 bytes; a range that does not start on a line
+// touches one more, which the neighbouring range brings in: the last one if the caller goes down
+// through the columns, the first one (`up`) if it goes up.
+__device__ __forceinline__ void prefetch_bias(const AttnExtras& ex, const uint8_t* rowp, int col0, int ncols,
+                                              bool up = false) {
   const int esize = ex.bias_f32 ? 4 : 2;
   const uint8_t* p = rowp + static_cast<int64_t>(col0) * esize;
-  for (int off = 0; off < ncols * esize; off += 128) prefetch_l2(p + off);
+  const int bytes = ncols * esize;
+  for (int off = 0; off < bytes; off += 128) prefetch_l2(p + (up ? min(off + 127, bytes - 1) : off));
 }
 
 constexpr int kTraceRoles = 3;   // softmax tile 0, softmax tile 1, MMA issuer

@@ -22,46 +22,51 @@
 
 namespace fo {
 
-// The walk of a warp whose query tile takes the steps `first` (0 or 1) to T - 1, two per key tile, on the
-// key tiles j0 to n - 1 of the ring (those before j0 belong to the CTA's other query tile).
+// The walk of a warp whose query tile takes the steps `first` (0 or 1) to `end` - 1, two per key tile, on
+// the key tiles j0 to j1 - 1 of the n that the ring carries (the others belong to the CTA's other query
+// tile).
 //   ops.wait(slot, parity)      blocks until that phase of the slot's "full" barrier is complete
 //   ops.ready(slot, parity)     the same without blocking
 //   ops.release(slot)           this warp's readers of the slot have all been issued
 //   ops.scores(t, slot)         issues the scores of step t, one of the first two, whose K tile is in `slot`
 //   ops.step(t, v_slot, k_slot) issues P V of step t and the scores of step t + 2 if there is one
 template <int kStages, class Ops>
-FO_RING_FN void walk_kv_ring(int j0, int n, int first, int T, const Ops& ops) {
+FO_RING_FN void walk_kv_ring(int j0, int j1, int n, int first, int end, const Ops& ops) {
   auto slot = [](int e) { return e % kStages; };
   auto parity = [](int e) { return static_cast<uint32_t>((e / kStages) & 1); };
-  for (int e = 0; e < 2 * j0; ++e) {
-    ops.wait(slot(e), parity(e));
-    ops.release(slot(e));
-  }
+  auto pass_over = [&](int e, int e_end) {
+    for (; e < e_end; ++e) {
+      ops.wait(slot(e), parity(e));
+      ops.release(slot(e));
+    }
+  };
+  pass_over(0, 2 * j0);
   ops.wait(slot(2 * j0), parity(2 * j0));
   ops.scores(first, slot(2 * j0));
-  if (first == 0 && T > 1) ops.scores(1, slot(2 * j0));
+  if (first == 0 && end > 1) ops.scores(1, slot(2 * j0));
   ops.release(slot(2 * j0));
-  if (first == 1 && T > 2) {
+  if (first == 1 && end > 2) {
     ops.wait(slot(2 * j0 + 2), parity(2 * j0 + 2));
     ops.scores(2, slot(2 * j0 + 2));
   }
   bool ready = false;  // looked at one step ahead, waited for only if that look failed
-  for (int t = first; t < T; ++t) {
+  for (int t = first; t < end; ++t) {
     const int j = (t >> 1) + j0;
     const int v = 2 * j + 1, k = v + 1;  // V of this step's key tile, K of the next
-    const bool k_next = j + 1 < n;
+    const bool k_next = j + 1 < j1;
     if (((t & 1) == 0 || t == first) && !ready) {
       ops.wait(slot(v), parity(v));
       if (k_next) ops.wait(slot(k), parity(k));
     }
     ready = false;
     ops.step(t, slot(v), slot(k));
-    if ((t & 1) == 1 || t + 1 == T) {
+    if ((t & 1) == 1 || t + 1 == end) {
       ops.release(slot(v));
       if (k_next) ops.release(slot(k));
-      if (t + 1 < T) ready = ops.ready(slot(v + 2), parity(v + 2)) && (!(j + 2 < n) || ops.ready(slot(k + 2), parity(k + 2)));
+      if (t + 1 < end) ready = ops.ready(slot(v + 2), parity(v + 2)) && (!(j + 2 < j1) || ops.ready(slot(k + 2), parity(k + 2)));
     }
   }
+  pass_over(2 * j1, 2 * n);
 }
 
 }  // namespace fo

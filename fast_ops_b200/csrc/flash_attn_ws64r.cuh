@@ -1,13 +1,17 @@
 // The 64-key forward kernel for attention with a bias (flash_attn_ws64.cuh has the roles, buffers and
-// barriers; this is the same pipeline): the key tiles are taken from the LAST to the FIRST.
+// barriers; this is the same pipeline): a CTA takes its key tiles from the last to the first, or from
+// the first to the last where the bias falls along the keys.
 //
-// A bias that grows with the key's position, as linear position biases do, raises the row maxima by
-// more than the rescaling threshold at almost every ascending step, and each time the step's
-// exponentials are taken again and O is rescaled in tensor memory; in descending order the first tile
-// sets the maximum.  B2 H16 S3072 D128 causal with linear biases: 221 us ascending, 147 descending;
-// key-padding bias B4 H16 S2048: 120 and 110.  A 16-bit matrix bias with 16-byte aligned rows is
-// fetched into registers a step ahead (together with the order: B2 H16 S2048 D64 with dropout 251 to
-// 183 us, D128 causal 99 to 85).
+// A bias that moves against the order raises the row maxima by more than the rescaling threshold at
+// almost every step, and each time the step's exponentials are taken again and O is rescaled in tensor
+// memory; with the order the first tile sets the maximum.  The CTA compares the bias of its first and
+// last key (read under the barrier set-up) and goes up if the first is larger by more than the
+// threshold; a bias that moves less than that never needs the choice.  us at B2 H16 S3072 with linear
+// biases, one order wrong and right: rising D128 causal 219 and 146, D64 284 and 179 without a mask;
+// falling D128 causal 181 and 149, D64 228 and 178.  Key padding (D128 causal 160 by the ascending
+// kernel of before) takes 144 either way.
+// A 16-bit matrix bias with 16-byte aligned rows is fetched into registers a step ahead.  B2 H16 S2048
+// against the ascending kernel: D64 170 to 129 us, with dropout 247 to 187, D128 causal 99 to 83.
 // It is a kernel of its own because the plain one does not bear the generalisation: compiled from
 // this source, without the bias, it took 341 us instead of 290 at B2 H32 S4096 D128 causal (the
 // order in which the assembler places the exponentials around the turn-taking barriers changes).
@@ -27,6 +31,13 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   constexpr int kTileBytes = Cfg::kTileBytes;
   constexpr int kStages = Cfg::kStages;
   constexpr int kBoxes = Cfg::kBoxes;
+  // Registers of the softmax warps and of the last four: 8 x kRegsSoftmax + 4 x 80 + 4 x kRegsRest are
+  // what the block was launched with, 16 x 128.  With dropout and a vector or 16-bit bias the second
+  // split and the hash index of a step formed in one register (kTight) avoid spills: B2 H16 S2048, vector
+  // bias D64 158 to 154 us, matrix bias D64 198 to 187, D128 225 to 203; the other forms measured slower
+  // with them (vector bias D128 S3072 198 to 229 us, fp32 matrix bias with dropout 259 to 285).
+  constexpr bool kTight = (kExt & kFwdDropout) != 0 && (kExt & kFwdMatBias32) == 0;
+  constexpr int kRegsSoftmax = kTight ? 184 : 192, kRegsRest = kTight ? 64 : 48;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -60,6 +71,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kOffMisc);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* skip = cta_abort + 1;
+  volatile int* ascending = cta_abort + 2;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -81,23 +93,23 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int vis1 = prm.causal ? min(prm.Sk, (2 * pair + 2) * kBlockM) : prm.Sk;
   const int n0 = (vis0 + kBlockN - 1) / kBlockN;
   const int n1 = (vis1 + kBlockN - 1) / kBlockN;
-  // The steps of a query tile are `first` to T - 1, two per key tile.  When the last key tile's upper
-  // half has no visible key, step 0 is left out (taken, with all its scores masked, it made 64 keys
-  // cost 38 us instead of 29 at B64 H12 D64, and 1088 keys 128 instead of 120 at B8 H16); its barrier
-  // phases are completed in the set-up, so that step numbers stand for buffers and phases as ever.
   const int T0 = 2 * n0, T1 = 2 * n1;  // T1 >= T0 >= 2
-  const int first0 = (vis0 + kStepN - 1) / kStepN & 1, first1 = (vis1 + kStepN - 1) / kStepN & 1;
-  // Tile 0 of the pair joins `skip0` steps after tile 1, which has the tiles next to the diagonal.
-  const int skip0 = (T1 - first1) - (T0 - first0);
-  // First key of step t.  A key tile's lower half comes before its upper half (in the tile on the
-  // diagonal more rows see it), and behind it if step 0 is left out.
-  auto step_key = [](int t, int first, int T) {
-    return T * kStepN - kBlockN * ((t >> 1) + 1) + ((t & 1) ^ first) * kStepN;
-  };
 
   if (tid == 0) {
     *cta_abort = 0;
+    // the ends of the bias over the keys that tile 0 sees (a matrix bias: in tile 1's first row); with a
+    // single key tile the order does not matter
+    float bias_first = 0.f, bias_last = 0.f;
+    if (n1 > 1) {
+      const int64_t row = min((2 * pair + 1) * kBlockM, prm.Sq - 1);
+      const uint8_t* const p = static_cast<const uint8_t*>(prm.ex.bias) +
+                               (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h + row * prm.ex.bias_stride_q) *
+                                   (prm.ex.bias_f32 ? 4 : 2);
+      bias_first = load_bias1<kBf16>(prm.ex, p, 0);
+      bias_last = load_bias1<kBf16>(prm.ex, p, vis0 - 1);
+    }
     *skip = *reinterpret_cast<volatile int*>(prm.device_status);
+    *ascending = bias_first - bias_last > kRescaleThreshold;
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(bar_kv_full + i, 1);
@@ -121,6 +133,25 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
   __syncthreads();
   if (*skip) return;  // another CTA already timed out: do nothing
+  const bool up = *ascending != 0;
+  // The steps of a query tile are `first` to `last`, two per key tile.  When the last key tile's upper
+  // half has no visible key, one is left out (taken, with all its scores masked, it made 64 keys cost
+  // 38 us instead of 29 at B64 H12 D64, and 1088 keys 128 instead of 120 at B8 H16): going up the very
+  // last one, going down step 0, whose barrier phases are then completed in the set-up, so that step
+  // numbers stand for buffers and phases as ever.
+  const int odd0 = (vis0 + kStepN - 1) / kStepN & 1, odd1 = (vis1 + kStepN - 1) / kStepN & 1;
+  const int first0 = up ? 0 : odd0, first1 = up ? 0 : odd1;
+  const int end0 = up ? T0 - odd0 : T0, end1 = up ? T1 - odd1 : T1;
+  // Tile 1 of the pair has up to two steps more than tile 0, those next to the diagonal: going down
+  // tile 0 joins `lead0` steps late, going up it ends `tail0` steps early.
+  const int extra = (end1 - first1) - (end0 - first0);
+  const int lead0 = up ? 0 : extra, tail0 = up ? extra : 0;
+  // First key of step t.  A key tile's lower half comes before its upper half (in the tile on the
+  // diagonal more rows see it), and behind it if step 0 is left out.
+  const int tile_dir = up ? kBlockN : -kBlockN;
+  auto step_key = [tile_dir](int t, int first, int key0) {
+    return key0 + (t >> 1) * tile_dir + ((t & 1) ^ first) * kStepN;
+  };
 
   // The first loads (Q and the first ring fill of K and V) need only the barriers: they go out
   // here, under the tensor-memory allocation, instead of after it.
@@ -131,7 +162,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const CUtensorMap* map = (i & 1) ? &tm_v : &tm_k;
     for (int c = 0; c < kBoxes; ++c)
       tma_load_4d(sKV + st * kTileBytes + c * kBoxBytes, map, bar_kv_full + st, c * kBoxCols,
-                  (n1 - 1 - (i >> 1)) * kBlockN, hk, b);
+                  (up ? i >> 1 : n1 - 1 - (i >> 1)) * kBlockN, hk, b);
   };
   if (warp == 13 && lane == 0) {
     mbar_arrive_expect_tx(bar_q_full, 2 * kTileBytes);
@@ -164,12 +195,13 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (warp < 8) {
     // ================================ softmax ================================
-    reg_alloc<192>();
+    reg_alloc<kRegsSoftmax>();
     const int s = warp >> 2;
     const int r = (warp & 3) * 32 + lane;
     const int q0 = (2 * pair + s) * kBlockM;
     const int row = q0 + r;
-    const int T_s = s ? T1 : T0, first = s ? first1 : first0;
+    const int first = s ? first1 : first0, end = s ? end1 : end0;
+    const int key0 = up ? 0 : (s ? n1 - 1 : n0 - 1) * kBlockN;  // first key of the first key tile
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS_tile = tmem_base + Cfg::kColS0 + s * kBlockN + lane_base;
     float* alpha_slot = s_alpha + s * 256 + r;
@@ -197,7 +229,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       if (vec_bias) {
         bias_vec = static_cast<const uint8_t*>(prm.ex.bias) +
                    (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h) * (prm.ex.bias_f32 ? 4 : 2);
-        const int col = T_s * kStepN - kBlockN + r;
+        const int col = key0 + r;
         bias_next = (col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
       }
     }
@@ -214,7 +246,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (ping_pong && s == 1) named_barrier_arrive(kTurn0, kTurnCount);
     // tile 0 takes and passes the turn for the steps that only tile 1 has
     if (ping_pong && s == 0)
-      for (int t = 0; t < skip0; ++t) {
+      for (int t = 0; t < lead0; ++t) {
         named_barrier_sync(kTurn0, kTurnCount);
         named_barrier_arrive(kTurn1, kTurnCount);
       }
@@ -225,7 +257,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     auto stage_vec_bias = [&](int tn) {
       const int j = tn >> 1;
       sb[(j & 1) * 128 + r] = bias_next;
-      const int col = T_s * kStepN - kBlockN * (j + 2) + r;  // of the key tile after this one (below 0: there is none)
+      const int col = key0 + (j + 1) * tile_dir + r;  // of the key tile after this one (there may be none)
       bias_next = (col >= 0 && col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
       // a buffer is rewritten two key tiles later, behind the barrier of the tile between
       named_barrier_sync(1 + s, 128);
@@ -241,7 +273,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     uint4 bias_raw[mat_bias16 ? 8 : 1];
     bool bias_held = false;
     auto fetch_mat_bias = [&](int tn) {
-      const int k0n = step_key(tn, first, T_s);
+      const int k0n = step_key(tn, first, key0);
       bias_held = bias_row != nullptr && prm.ex.bias_vec && k0n + kStepN <= prm.Sk;
       if (bias_held) {
         const uint4* const p = reinterpret_cast<const uint4*>(bias_row + static_cast<int64_t>(k0n) * 2);
@@ -249,9 +281,15 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         for (int i = 0; i < (mat_bias16 ? 8 : 1); ++i) bias_raw[i] = __ldg(p + i);
       }
     };
+    auto add_bias2 = [&](int c, int i, float2 bias2) {  // scores i and i + 1 of chunk c, scaled, plus their bias
+      const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])),
+                                  make_float2(prm.scale_log2, prm.scale_log2), bias2);
+      sr[c][i] = __float_as_uint(x.x);
+      sr[c][i + 1] = __float_as_uint(x.y);
+    };
     // Waits for those loads and applies bias and masks in place.
     auto prep_loads = [&](int tn) {
-      const int k0n = step_key(tn, first, T_s);
+      const int k0n = step_key(tn, first, key0);
       const bool need_mask = (k0n + kStepN > prm.Sk) || (prm.causal && k0n + kStepN - 1 > q0);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -263,10 +301,8 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
               const float4 v4 = bv[i >> 2];  // the same address in every thread: a broadcast
-              sr[c][i + 0] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 0]), prm.scale_log2, v4.x));
-              sr[c][i + 1] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 1]), prm.scale_log2, v4.y));
-              sr[c][i + 2] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 2]), prm.scale_log2, v4.z));
-              sr[c][i + 3] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 3]), prm.scale_log2, v4.w));
+              add_bias2(c, i, make_float2(v4.x, v4.y));
+              add_bias2(c, i + 2, make_float2(v4.z, v4.w));
             }
           }
           if constexpr (mat_bias) {
@@ -279,17 +315,16 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int y = 0; y < 4; ++y) {
-                  const float2 f = unpack2<kBf16>(w[y]);
-                  bb[8 * i + 2 * y] = f.x * kLog2e;
-                  bb[8 * i + 2 * y + 1] = f.y * kLog2e;
+                  const float2 f = __fmul2_rn(unpack2<kBf16>(w[y]), make_float2(kLog2e, kLog2e));
+                  bb[8 * i + 2 * y] = f.x;
+                  bb[8 * i + 2 * y + 1] = f.y;
                 }
               }
             } else {
               load_bias32<kBf16, mat_bias16 ? kBias16 : kBias32>(prm.ex, bias_row, k0n + c * 32, prm.Sk, bb);
             }
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              sr[c][i] = __float_as_uint(fmaf(__uint_as_float(sr[c][i]), prm.scale_log2, bb[i]));
+            for (int i = 0; i < 32; i += 2) add_bias2(c, i, make_float2(bb[i], bb[i + 1]));
           }
         }
         if (need_mask) {
@@ -338,9 +373,10 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // exponentials taken again.  Each iteration then fetches step t + 1 (whose S the tensor core
     // finished meanwhile) behind the P stores, so that the latencies of the loads, of the P store
     // and of the barriers overlap instead of adding up.
-    for (int t = first; t < T_s; ++t) {
+    for (int t = first; t < end; ++t) {
       const int u = t & 1;
-      const int k0 = step_key(t, first, T_s);
+      const int k0 = step_key(t, first, key0);
+      const uint32_t drop_idx = drop_row + (kTight ? static_cast<uint32_t>(k0) : 0u);
       const uint32_t tS = tS_tile + u * kStepN;
       float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
       if (ping_pong) named_barrier_sync_dep(s ? kTurn1 : kTurn0, kTurnCount, neg_m);  // exponentials start after this
@@ -348,7 +384,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const float2 sc2 = make_float2(exp_scale, exp_scale);
       float2 acc0, acc1;
       uint32_t pr[2][16];
-      const bool more = t + 1 < T_s;
+      const bool more = t + 1 < end;
       bool s_next_ready = false;
       float mxa = -INFINITY, mxb = -INFINITY;
       // P = exp2(S * scale - reference) for the whole step; `first` is the pass that also passes
@@ -385,7 +421,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               // dropped elements leave the row sum untouched and enter P V as zeros; the factor
               // 1 / (1 - p) is applied once, to O, in the epilogue
               if (has_drop) {
-                const uint32_t idx = drop_row + static_cast<uint32_t>(k0 + c * 32 + 2 * q);
+                const uint32_t idx = drop_idx + static_cast<uint32_t>((kTight ? 0 : k0) + c * 32 + 2 * q);
                 if (dropout_hash(idx, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.x = 0.f;
                 if (dropout_hash(idx + 1u, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.y = 0.f;
               }
@@ -421,9 +457,9 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if constexpr (kExt != 0) {
           if (vec_bias && u == 1) stage_vec_bias(t + 1);
           if constexpr (mat_bias16) fetch_mat_bias(t + 1);
-          if (mat_bias && bias_row != nullptr && t + 2 < T_s) {
-            const int c0 = step_key(t + 2, first, T_s);
-            if (c0 < prm.Sk) prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0));
+          if (mat_bias && bias_row != nullptr && t + 2 < end) {
+            const int c0 = step_key(t + 2, first, key0);
+            prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0), up);
           }
         }
         if (!s_next_ready)
@@ -441,6 +477,15 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       if (more) prep_loads(t + 1);
       if ((warp & 3) == 0) trace_event(prm, s, t, 5);
     }
+    // Tile 0 keeps taking and passing the turn for the steps that only tile 1 still has, one at a time
+    // (arrivals sent ahead of the other tile's waits would complete a barrier phase on their own and
+    // strand it).  Tile 1's very last arrival finds nobody waiting: the CTA ends with that barrier half
+    // counted, which is harmless.
+    if (ping_pong && s == 0)
+      for (int t = 0; t < tail0; ++t) {
+        named_barrier_sync(kTurn0, kTurnCount);
+        named_barrier_arrive(kTurn1, kTurnCount);
+      }
     s_final[s * 256 + r] = l_run;
     s_final[s * 256 + 128 + r] = m_run;
     mbar_arrive(bar_final + s);
@@ -485,12 +530,12 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             (l_run > 0.f) ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
       }
     };
-    for (int g = first1; g < T1; ++g) {
+    for (int g = first1; g < end1; ++g) {
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const int first = s ? first1 : first0;
-        const int t = s ? g : g - first1 - skip0 + first0;
-        if (t < first) continue;
+        const int t = s ? g : g - first1 - lead0 + first0;
+        if (t < first || t >= (s ? end1 : end0)) continue;
         mbar_wait(bar_corr + 2 * s + (t & 1), (t >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_SOFTMAX);
         const float alpha = s_alpha[s * 256 + (t & 1) * 128 + r];
         if (t > first && __any_sync(0xffffffffu, alpha != 1.f)) {
@@ -520,7 +565,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     epilogue(0);
     epilogue(1);
   } else {
-    reg_dealloc<48>();
+    reg_dealloc<kRegsRest>();
     if (warp == 12 || warp == 14) {
       // ================================ MMA issuers ================================
       // One warp per query tile (12: tile 0, 14: tile 1).  The tensor core's instruction queue
@@ -530,7 +575,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // other, and nothing has to: each tile owns its S / P buffers and its O accumulator, and a
       // K/V ring slot is released by both warps (bar_kv_empty counts two arrivals).
       const int s = (warp == 14) ? 1 : 0;
-      const int T_s = s ? T1 : T0, first = s ? first1 : first0;
+      const int first = s ? first1 : first0, end = s ? end1 : end0;
       constexpr uint32_t idesc_qk = make_idesc(kBf16, kBlockM, kStepN, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc(kBf16, kBlockM, D, 0, 1);
       // Everything below is warp-uniform; only the tcgen05 instructions themselves are issued by
@@ -586,16 +631,16 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if (s == 0) trace_event(prm, 2, t, 1);
         issue_pv(u, v_slot, t > first);
         tcgen05_commit_elect(bar_o_full + s);
-        if (t + 1 == T_s) tcgen05_commit_elect(bar_o_done + s);
+        if (t + 1 == end) tcgen05_commit_elect(bar_o_done + s);
         if (s == 0) trace_event(prm, 2, t, 2);
         // step t + 2 goes into the buffer that P(s, t) is being read from; the tensor core runs
         // one thread's instructions in order, so the read comes first
-        if (t + 2 < T_s) {
+        if (t + 2 < end) {
           issue_s(u, k_slot);
           tcgen05_commit_elect(bar_s_full + 2 * s + u);
         }
         if (s == 0) trace_event(prm, 2, t, 3);
-        p_ready = (t + 1 < T_s) && mbar_test_wait(bar_p_full + 2 * s + (u ^ 1), ((t + 1) >> 1) & 1);
+        p_ready = (t + 1 < end) && mbar_test_wait(bar_p_full + 2 * s + (u ^ 1), ((t + 1) >> 1) & 1);
       };
       mbar_wait(bar_q_full, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_TMA);
       struct {
@@ -605,8 +650,8 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         decltype(scores) scores;
         decltype(step) step;
       } const ops{wait_kv, kv_ready, release_kv, scores, step};
-      // the ring's first key tile is read by tile 1 alone if tile 0 joins a whole key tile later
-      walk_kv_ring<kStages>(s ? 0 : n1 - n0, n1, first, T_s, ops);
+      const int j0 = s || up ? 0 : n1 - n0;  // first of the ring's key tiles that this query tile reads
+      walk_kv_ring<kStages>(j0, j0 + (s ? n1 : n0), n1, first, end, ops);
     } else if (warp == 13) {
       // ================================ TMA producer ================================
       const bool issuer = lane == 0;

@@ -6,6 +6,7 @@ import torch
 
 import fast_ops_b200._lib as L
 import oracle
+from fast_ops_b200.flash_attention import flash_attention_forward
 from helpers import attention_dout, attention_inputs
 from test_gpu_5_attention_bias_dropout import check, run_case
 
@@ -65,3 +66,21 @@ def test_bias_that_moves_the_maximum(cuda_device, Sq, Sk, causal, kind, D, dtype
     out, lse_o, dq, dk, dv = oracle.attention_ex(q, k, v, bias=bias, keep_mask=keep, dropout_p=p, causal=causal, dout=dout)
     check(got, same, (out, dq, dk, dv), f"{kind} {Sq}x{Sk}")
     assert torch.allclose(lse.cpu(), lse_o, atol=2e-3, rtol=1e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("form", ["vector", "matrix"])
+def test_rows_masked_by_a_large_finite_bias(cuda_device, dtype, form):
+    """Every key of a row at -1e9: in fp32 the scores vanish beside it, so the row is the mean of V."""
+    B, H, Sq, Sk, D = 1, 2, 300, 450, 64
+    q, k, v = (t.to(cuda_device) for t in attention_inputs(5, B, H, Sq, Sk, D, dtype))
+    bias = torch.full((1, 1, 1 if form == "vector" else Sq, Sk), -1e9, device=cuda_device)
+    L.attn_configure(impl="ws64")
+    try:
+        o = flash_attention_forward(q, k, v, bias=bias)
+    finally:
+        L.attn_configure(impl="auto")
+    want = v.double().mean(2, keepdim=True).expand_as(o)
+    # the weights are exactly 1: fp32 sums of Sk terms below 5, one rounding of the result
+    eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert ((o.double() - want).abs() <= eps * want.abs() + 1e-5).all()

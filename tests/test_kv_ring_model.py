@@ -18,20 +18,20 @@ RECORDER = r"""
 #include <cstdlib>
 #include "flash_attn_ring.h"
 struct Ops {
-  int T;
+  int end;
   void wait(int slot, uint32_t parity) const { printf("w %d %u\n", slot, parity); }
   bool ready(int, uint32_t) const { return false; }
   void release(int slot) const { printf("r %d\n", slot); }
   void scores(int t, int slot) const { printf("k %d %d\n", t, slot); }
   void step(int t, int v_slot, int k_slot) const {
     printf("v %d %d\n", t, v_slot);
-    if (t + 2 < T) printf("k %d %d\n", t + 2, k_slot);
+    if (t + 2 < end) printf("k %d %d\n", t + 2, k_slot);
   }
 };
 int main(int, char** a) {
-  const int stages = atoi(a[1]), j0 = atoi(a[2]), n = atoi(a[3]), first = atoi(a[4]), T = atoi(a[5]);
-  if (stages == 4) fo::walk_kv_ring<4>(j0, n, first, T, Ops{T});
-  else fo::walk_kv_ring<6>(j0, n, first, T, Ops{T});
+  const int stages = atoi(a[1]), j0 = atoi(a[2]), j1 = atoi(a[3]), n = atoi(a[4]), first = atoi(a[5]), end = atoi(a[6]);
+  if (stages == 4) fo::walk_kv_ring<4>(j0, j1, n, first, end, Ops{end});
+  else fo::walk_kv_ring<6>(j0, j1, n, first, end, Ops{end});
 }
 """
 
@@ -44,11 +44,11 @@ def recorder(tmp_path_factory):
         f.write(RECORDER)
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, src, "-o", exe], check=True)
 
-    def record(stages, n, halves):
-        """The walk of a query tile that sees `halves` half key tiles, in a ring of n key tiles."""
-        first, T = halves % 2, (halves + 1) // 2 * 2
-        j0 = n - T // 2
-        args = [stages, j0, n, first, T]
+    def record(stages, n, halves, up):
+        """The walk, up or down, of a query tile that sees `halves` half key tiles, in a ring of n key tiles."""
+        own = (halves + 1) // 2
+        j0 = 0 if up else n - own
+        args = [stages, j0, j0 + own, n, 0 if up else halves % 2, halves if up else 2 * own]
         out = subprocess.run([exe, *map(str, args)], check=True, capture_output=True, text=True).stdout
         ops = []
         for line in out.splitlines():
@@ -119,10 +119,11 @@ def run(stages, entries, warps, rng, order):
 @pytest.mark.parametrize("order", ["random", "reversed"])
 @pytest.mark.parametrize("seen0,seen1", [(1, 1), (2, 2), (2, 3), (2, 4), (3, 3), (4, 4), (4, 5), (4, 6), (5, 5), (6, 7),
                                          (6, 8), (8, 10), (11, 11), (12, 14), (17, 17), (18, 20), (19, 19)])
-def test_every_read_finds_its_entry(recorder, stages, order, seen0, seen1):
+@pytest.mark.parametrize("up", [False, True], ids=["descending", "ascending"])
+def test_every_read_finds_its_entry(recorder, stages, order, seen0, seen1, up):
     """Query tile 0 sees seen0 half key tiles, tile 1 seen1 (up to two more under a causal mask)."""
     n1 = (seen1 + 1) // 2
-    warps = [recorder(stages, n1, seen) for seen in (seen0, seen1)]
+    warps = [recorder(stages, n1, seen, up) for seen in (seen0, seen1)]
     for warp, seen in zip(warps, (seen0, seen1)):
         assert sum(op[0] == "read" for op in warp) == 2 * seen  # K and V of every step
         assert sum(op[0] == "release" for op in warp) == 2 * n1
@@ -132,7 +133,7 @@ def test_every_read_finds_its_entry(recorder, stages, order, seen0, seen1):
 
 def test_the_model_sees_a_wait_that_is_missing(recorder):
     """Passing over the first key tile without waiting for it lets a warp take entry 4 for loaded."""
-    warps = [recorder(4, 3, seen) for seen in (4, 6)]
+    warps = [recorder(4, 3, seen, False) for seen in (4, 6)]
     assert warps[0][:4] == [("wait", 0, 0), ("release", 0), ("wait", 1, 0), ("release", 1)]
     del warps[0][2], warps[0][0]
     with pytest.raises(AssertionError, match="reads entry"):
