@@ -353,11 +353,14 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
     // causal: S=16384 1.11 against 1.02 PFLOP/s, S=4096 0.98 against 0.82, GPT-2-small shape
     // 0.29 against 0.21); the 128-key kernel stays selectable.
     impl = AttnImpl::kWarpSpecialized64;
-    // one exception, also measured: with a bias and no dropout, over a long key range, the
-    // 128-key kernel is about 7 % ahead (0.79 against 0.73 PFLOP/s at S=16384)
+    // one exception, also measured: at head_dim <= 64 with a vector bias and no dropout, over a long key
+    // range, the 128-key kernel is ahead (us, 128-key and 64-key kernel, no mask: Sk=6272 325 and 346,
+    // 8192 532 and 591, B1 H8 Sk=16384 1031 and 1162, causal 533 and 543; a rising bias 372 and 346, 595 and
+    // 591, 1143 and 1161).  Not at head_dim 128 (Sk=8192 735 and 673, rising 816 and 672, causal 432 and
+    // 349) and not with a matrix bias (D64 Sk=8192 1237 and 933, D128 1558 and 994).
     const int n_kv = (Sk + kBlockN - 1) / kBlockN;
-    const bool bias_only = ext && ex->bias != nullptr && !ex->dropout;
-    if (bias_only && (causal ? (n_kv + 1) / 2 : n_kv) > 48) impl = AttnImpl::kWarpSpecialized;
+    const bool vec_bias_only = ext && ex->bias != nullptr && ex->bias_stride_q == 0 && !ex->dropout;
+    if (vec_bias_only && Dk == 64 && (causal ? (n_kv + 1) / 2 : n_kv) > 48) impl = AttnImpl::kWarpSpecialized;
     // Plain attention where a CTA's life is short or the grid is small runs one query tile per CTA
     // and two CTAs per SM (measured, bf16 causal, same box: D=64 8 to 28 % ahead at every length
     // from 512 to 8192; D=128 3 % ahead at S=1024, 5 % behind at S=2048, 10 % behind at S=16384,

@@ -155,11 +155,13 @@ def _bias_of(code, B, H, Sq, Sk, seed, dtype=torch.float32):
     return bias
 
 
-def test_long_key_range_with_vector_bias_takes_the_128_key_kernel(cuda_device):
-    """Nothing forced: a bias without dropout over more than 48 key tiles is where the library
-    switches from the 64-key to the 128-key forward kernel.  Sk = 6272 is 49 tiles, not causal."""
+@pytest.mark.parametrize("D", [64, 128])
+def test_long_key_range_with_vector_bias(cuda_device, D):
+    """Nothing forced: a vector bias without dropout over more than 48 key tiles is where the library
+    switches from the 64-key to the 128-key forward kernel at head_dim 64 (and stays with the 64-key
+    kernel at 128).  Sk = 6272 is 49 tiles, not causal."""
     L.attn_configure(impl="auto")
-    B, H, Sq, Sk, D = 1, 1, 384, 6272, 128
+    B, H, Sq, Sk = 1, 1, 384, 6272
     q, k, v = attention_inputs(77, B, H, Sq, Sk, D, torch.bfloat16)
     dout = attention_dout(78, B, H, Sq, D, torch.bfloat16)
     bias = _bias_of("1h1k", B, H, Sq, Sk, 79)
