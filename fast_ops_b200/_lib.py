@@ -150,12 +150,11 @@ def current_stream_ptr(device) -> int:
         _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
             lambda i: torch.cuda.current_stream(i).cuda_stream)
     if type(device) is not int:
-        index = device.index
-        if index is None:
-            import torch
+        import torch
 
-            index = torch.cuda.current_device()
-        device = index
+        device = device.index if isinstance(device, torch.device) else int(device)
+        if device is None:
+            device = torch.cuda.current_device()
     return _raw_stream(device)
 
 

@@ -69,3 +69,13 @@ def test_attention_options_are_validated_without_a_gpu():
     assert lib.fo_attn_configure(-1, -1, -2) == -1 and b"head_group" in lib.fo_last_error()
     L.attn_configure(impl="ws", ping_pong=False, head_group=3)
     L.attn_configure(impl="auto", ping_pong=True, head_group=0)
+
+
+def test_stream_accessor_takes_devices_and_indices(monkeypatch):
+    """A torch.device or anything that converts to an index, as integers of numpy do."""
+    import numpy as np
+    import torch
+
+    monkeypatch.setattr(L, "_raw_stream", lambda index: 100 + index)
+    for device in (2, np.int64(2), torch.device("cuda", 2)):
+        assert L.current_stream_ptr(device) == 102
