@@ -372,11 +372,12 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
   }
   const int mode = ext ? ((prm.ex.bias != nullptr ? 1 : 0) | (prm.ex.dropout ? 2 : 0)) : 0;
   // bias and dropout exist in the warp-specialised kernels only
-#define FO_WS_MODE(LAUNCH, M)                                                                          \
-  if (mode == M) {                                                                                     \
+#define FO_WS_FORM(FORM, LAUNCH, M)                                                                    \
+  if (FORM == M) {                                                                                     \
     if (Dk == 128) return bf16 ? fo::LAUNCH<128, true, M>(tq, tk, tv, prm, s) : fo::LAUNCH<128, false, M>(tq, tk, tv, prm, s); \
     return bf16 ? fo::LAUNCH<64, true, M>(tq, tk, tv, prm, s) : fo::LAUNCH<64, false, M>(tq, tk, tv, prm, s);                 \
   }
+#define FO_WS_MODE(LAUNCH, M) FO_WS_FORM(mode, LAUNCH, M)
   if (impl == AttnImpl::kShort64 && mode == 0) {
     // one query tile per CTA, two CTAs per SM: K and V are loaded in 64-key halves
     CUtensorMap tkh, tvh;
@@ -396,18 +397,15 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
       return bf16 ? fo::launch_ws64<128, true, 0, 96>(tq, tk, tv, prm, s) : fo::launch_ws64<128, false, 0, 96>(tq, tk, tv, prm, s);
     FO_WS_MODE(launch_ws64, 0)
     FO_WS_MODE(launch_ws64, 2)
-    // with a bias: the kernel that takes the keys in descending order, vector and matrix compiled apart
-    const int drop = mode & fo::kFwdDropout;
-    {
-      const int form = prm.ex.bias_stride_q == 0 ? fo::kFwdVecBias : prm.ex.bias_f32 ? fo::kFwdMatBias32 : fo::kFwdMatBias;
-      const int mode = form | drop;
-      FO_WS_MODE(launch_ws64r, 1)
-      FO_WS_MODE(launch_ws64r, 3)
-      FO_WS_MODE(launch_ws64r, 4)
-      FO_WS_MODE(launch_ws64r, 6)
-      FO_WS_MODE(launch_ws64r, 8)
-      FO_WS_MODE(launch_ws64r, 10)
-    }
+    // with a bias: the kernel that chooses the order of the keys, vector, 16-bit and fp32 matrix compiled apart
+    const int bias_form = prm.ex.bias_stride_q == 0 ? fo::kFwdVecBias : prm.ex.bias_f32 ? fo::kFwdMatBias32 : fo::kFwdMatBias;
+    const int form = bias_form | (mode & fo::kFwdDropout);
+    FO_WS_FORM(form, launch_ws64r, 1)
+    FO_WS_FORM(form, launch_ws64r, 3)
+    FO_WS_FORM(form, launch_ws64r, 4)
+    FO_WS_FORM(form, launch_ws64r, 6)
+    FO_WS_FORM(form, launch_ws64r, 8)
+    FO_WS_FORM(form, launch_ws64r, 10)
   }
   if (impl != AttnImpl::kSimple || mode != 0) {
     FO_WS_MODE(launch_ws, 0)
@@ -416,6 +414,7 @@ static int attn_fwd_impl(const void* q, const void* k, const void* v, void* o, f
     FO_WS_MODE(launch_ws, 3)
   }
 #undef FO_WS_MODE
+#undef FO_WS_FORM
   if (Dk == 128) return bf16 ? launch_simple<128, true>(tq, tk, tv, prm, s) : launch_simple<128, false>(tq, tk, tv, prm, s);
   return bf16 ? launch_simple<64, true>(tq, tk, tv, prm, s) : launch_simple<64, false>(tq, tk, tv, prm, s);
 }

@@ -36,12 +36,14 @@ struct Ws64Config : WsConfig<D> {
   static constexpr int kSmemBytes = kOffMisc + 64 + 1024 /* alignment slack */;
 };
 
+// kExt: 0 or kFwdDropout (with a bias flash_attn_ws64r.cuh is the kernel).
 // kMma: the head_dim the matmuls compute, at most the tiles' width D (the columns between are zeros;
 // B1 H48 Sq1000 Sk1531 D80: 57 to 55.7 us with 96 instead of 128 columns computed).
 template <int D, bool kBf16, int kExt, int kMma = D>
 __global__ void __launch_bounds__(512, 1)
 attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const AttnParams prm) {
+  static_assert(kExt == 0 || kExt == kFwdDropout, "a bias runs in attn_fwd_ws64r_kernel");
   using Cfg = Ws64Config<D>;
   constexpr int kTileBytes = Cfg::kTileBytes;
   constexpr int kStages = Cfg::kStages;
@@ -53,7 +55,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint8_t* sKV = smem + Cfg::kOffKV;  // kStages tiles
   float* s_alpha = reinterpret_cast<float*>(smem + Cfg::kOffAlpha);
   float* s_final = reinterpret_cast<float*>(smem + Cfg::kOffFinal);
-  float* s_bias = reinterpret_cast<float*>(smem + Cfg::kOffBias);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBars);
   uint64_t* bar_q_full = bars;                     // TMA -> MMA
   uint64_t* bar_kv_full = bars + 1;                // [kStages] TMA -> MMA
@@ -170,32 +171,12 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t tS_tile = tmem_base + Cfg::kColS0 + s * kBlockN + lane_base;
     float* alpha_slot = s_alpha + s * 256 + r;
     float m_run = -INFINITY, l_run = 0.f;
-    constexpr bool has_bias = (kExt & 1) != 0;
-    constexpr bool has_drop = (kExt & 2) != 0;
-    const uint8_t* bias_row = nullptr;
+    constexpr bool has_drop = kExt == kFwdDropout;
     uint32_t drop_row = 0;
-    if constexpr (kExt != 0) {
-      if (has_bias && row < prm.Sq)
-        bias_row = static_cast<const uint8_t*>(prm.ex.bias) +
-                   (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h + static_cast<int64_t>(row) * prm.ex.bias_stride_q) *
-                       (prm.ex.bias_f32 ? 4 : 2);
+    if constexpr (has_drop)
       drop_row = prm.ex.drop_base + static_cast<uint32_t>(bh) * static_cast<uint32_t>(prm.Sq) * static_cast<uint32_t>(prm.Sk) +
                  static_cast<uint32_t>(row) * static_cast<uint32_t>(prm.Sk);
-    }
-    // with a bias the scores are scaled when the bias is added, not in the exponent
-    const float exp_scale = has_bias ? 1.f : prm.scale_log2;
-    // a row-independent bias goes through shared memory, fetched one 128-key tile ahead
-    const bool vec_bias = has_bias && prm.ex.bias_stride_q == 0;
-    const uint8_t* bias_vec = nullptr;
-    float* sb = s_bias + s * 256;
-    float bias_next = 0.f;
-    if constexpr (kExt != 0) {
-      if (vec_bias) {
-        bias_vec = static_cast<const uint8_t*>(prm.ex.bias) +
-                   (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h) * (prm.ex.bias_f32 ? 4 : 2);
-        bias_next = (r < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, r) : 0.f;
-      }
-    }
+    const float exp_scale = prm.scale_log2;
 
     // S of the next step is normally complete long before it is needed: polled once while the
     // current step's exponentials are in flight, waited on only if that poll failed
@@ -208,23 +189,14 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const bool ping_pong = prm.ping_pong != 0;
     if (ping_pong && s == 1) named_barrier_arrive(kTurn0, kTurnCount);
 
-    uint32_t sr[2][32];  // scores of the current step (scaled and biased already when there is a bias)
+    uint32_t sr[2][32];  // scores of the current step
 
-    // Stages the row-independent bias of the key tile that step `tn` (even) starts.
-    auto stage_vec_bias = [&](int tn) {
-      const int j = tn >> 1;
-      sb[(j & 1) * 128 + r] = bias_next;
-      const int col = tn * kStepN + kBlockN + r;
-      bias_next = (col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
-      // a buffer is rewritten two key tiles later, behind the barrier of the tile between
-      named_barrier_sync(1 + s, 128);
-    };
     // Issues the tensor-memory loads of step tn's scores (S must be complete).
     auto issue_load = [&](int tn, int c) {
       const uint32_t tSn = tS_tile + (tn & 1) * kStepN;
       tmem_ld32(tSn + c * 32, sr[c]);
     };
-    // Waits for those loads and applies bias and masks in place.
+    // Waits for those loads and applies the masks in place.
     auto prep_loads = [&](int tn) {
       const int k0n = tn * kStepN;
       const bool need_mask = (k0n + kStepN > prm.Sk) || (prm.causal && k0n + kStepN - 1 > q0);
@@ -232,25 +204,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       for (int c = 0; c < 2; ++c) {
         tmem_ld_wait(sr[c]);
         if ((warp & 3) == 0 && tn > 0) trace_event(prm, s, tn - 1, c == 0 ? 1 : 4);  // loads in
-        if constexpr (kExt != 0) {
-          if (vec_bias) {
-            const float4* bv = reinterpret_cast<const float4*>(sb + ((tn >> 1) & 1) * 128 + (tn & 1) * kStepN + c * 32);
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 v4 = bv[i >> 2];  // the same address in every thread: a broadcast
-              sr[c][i + 0] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 0]), prm.scale_log2, v4.x));
-              sr[c][i + 1] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 1]), prm.scale_log2, v4.y));
-              sr[c][i + 2] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 2]), prm.scale_log2, v4.z));
-              sr[c][i + 3] = __float_as_uint(fmaf(__uint_as_float(sr[c][i + 3]), prm.scale_log2, v4.w));
-            }
-          } else if (has_bias) {
-            float bb[32];
-            load_bias32<kBf16>(prm.ex, bias_row, k0n + c * 32, prm.Sk, bb);
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              sr[c][i] = __float_as_uint(fmaf(__uint_as_float(sr[c][i]), prm.scale_log2, bb[i]));
-          }
-        }
         if (need_mask) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -278,9 +231,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     };
 
     // prologue: scores of step 0; their row maximum is the first reference maximum
-    if constexpr (kExt != 0) {
-      if (vec_bias) stage_vec_bias(0);
-    }
     mbar_wait(bar_s_full + 2 * s, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
     tcgen05_fence_after_sync();
     issue_load(0, 0);
@@ -339,14 +289,12 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             if (first) {
               if (q & 1) mxb = max3(mxb, a, b); else mxa = max3(mxa, a, b);
             }
-            if constexpr (kExt != 0) {
+            if constexpr (has_drop) {
               // dropped elements leave the row sum untouched and enter P V as zeros; the factor
               // 1 / (1 - p) is applied once, to O, in the epilogue
-              if (has_drop) {
-                const uint32_t idx = drop_row + static_cast<uint32_t>(k0 + c * 32 + 2 * q);
-                if (dropout_hash(idx, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.x = 0.f;
-                if (dropout_hash(idx + 1u, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.y = 0.f;
-              }
+              const uint32_t idx = drop_row + static_cast<uint32_t>(k0 + c * 32 + 2 * q);
+              if (dropout_hash(idx, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.x = 0.f;
+              if (dropout_hash(idx + 1u, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.y = 0.f;
             }
             pr[c][q] = pack2<kBf16>(x.x, x.y);
           }
@@ -376,13 +324,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // S of step t + 1 was issued when P of step t - 1 was handed over: complete by now as a
         // rule.  Its loads go out behind the P stores; the score registers are free, everything
         // of step t is in pr.
-        if constexpr (kExt != 0) {
-          if (vec_bias && u == 1) stage_vec_bias(t + 1);
-          if (!vec_bias && bias_row != nullptr) {
-            const int c0 = k0 + kStepN;
-            prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0));
-          }
-        }
         if (!s_next_ready)
           mbar_wait(bar_s_full + 2 * s + (u ^ 1), ((t + 1) >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
         tcgen05_fence_after_sync();

@@ -210,28 +210,24 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     constexpr bool mat_bias = mat_bias16 || (kExt & kFwdMatBias32) != 0;
     constexpr bool has_drop = (kExt & kFwdDropout) != 0;
     const uint8_t* bias_row = nullptr;
-    uint32_t drop_row = 0;
-    if constexpr (kExt != 0) {
-      if (mat_bias && row < prm.Sq)
-        bias_row = static_cast<const uint8_t*>(prm.ex.bias) +
-                   (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h + static_cast<int64_t>(row) * prm.ex.bias_stride_q) *
-                       (prm.ex.bias_f32 ? 4 : 2);
-      drop_row = prm.ex.drop_base + static_cast<uint32_t>(bh) * static_cast<uint32_t>(prm.Sq) * static_cast<uint32_t>(prm.Sk) +
-                 static_cast<uint32_t>(row) * static_cast<uint32_t>(prm.Sk);
-    }
-    // with a bias the scores are scaled when the bias is added, not in the exponent
+    if (mat_bias && row < prm.Sq)
+      bias_row = static_cast<const uint8_t*>(prm.ex.bias) +
+                 (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h + static_cast<int64_t>(row) * prm.ex.bias_stride_q) *
+                     (prm.ex.bias_f32 ? 4 : 2);
+    const uint32_t drop_row = prm.ex.drop_base +
+                              static_cast<uint32_t>(bh) * static_cast<uint32_t>(prm.Sq) * static_cast<uint32_t>(prm.Sk) +
+                              static_cast<uint32_t>(row) * static_cast<uint32_t>(prm.Sk);
+    // the scores are scaled when the bias is added, not in the exponent
     const float exp_scale = 1.f;
     // a row-independent bias goes through shared memory, fetched one 128-key tile ahead
     const uint8_t* bias_vec = nullptr;
     float* sb = s_bias + s * 256;
     float bias_next = 0.f;
-    if constexpr (kExt != 0) {
-      if (vec_bias) {
-        bias_vec = static_cast<const uint8_t*>(prm.ex.bias) +
-                   (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h) * (prm.ex.bias_f32 ? 4 : 2);
-        const int col = key0 + r;
-        bias_next = (col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
-      }
+    if constexpr (vec_bias) {
+      bias_vec = static_cast<const uint8_t*>(prm.ex.bias) +
+                 (b * prm.ex.bias_stride_b + h * prm.ex.bias_stride_h) * (prm.ex.bias_f32 ? 4 : 2);
+      const int col = key0 + r;
+      bias_next = (col < prm.Sk) ? load_bias1<kBf16>(prm.ex, bias_vec, col) : 0.f;
     }
 
     // S of the next step is normally complete long before it is needed: polled once while the
@@ -295,37 +291,35 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       for (int c = 0; c < 2; ++c) {
         tmem_ld_wait(sr[c]);
         if ((warp & 3) == 0 && tn > 0) trace_event(prm, s, tn - 1, c == 0 ? 1 : 4);  // loads in
-        if constexpr (kExt != 0) {
-          if (vec_bias) {
-            const float4* bv = reinterpret_cast<const float4*>(sb + ((tn >> 1) & 1) * 128 + ((tn & 1) ^ first) * kStepN + c * 32);
+        if constexpr (vec_bias) {
+          const float4* bv = reinterpret_cast<const float4*>(sb + ((tn >> 1) & 1) * 128 + ((tn & 1) ^ first) * kStepN + c * 32);
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 v4 = bv[i >> 2];  // the same address in every thread: a broadcast
-              add_bias2(c, i, make_float2(v4.x, v4.y));
-              add_bias2(c, i + 2, make_float2(v4.z, v4.w));
-            }
+          for (int i = 0; i < 32; i += 4) {
+            const float4 v4 = bv[i >> 2];  // the same address in every thread: a broadcast
+            add_bias2(c, i, make_float2(v4.x, v4.y));
+            add_bias2(c, i + 2, make_float2(v4.z, v4.w));
           }
-          if constexpr (mat_bias) {
-            float bb[32];
-            if (mat_bias16 && bias_held) {
-              constexpr float kLog2e = 1.4426950408889634f;
+        }
+        if constexpr (mat_bias) {
+          float bb[32];
+          if (mat_bias16 && bias_held) {
+            constexpr float kLog2e = 1.4426950408889634f;
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const uint4 v = bias_raw[mat_bias16 ? c * 4 + i : 0];
-                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            for (int i = 0; i < 4; ++i) {
+              const uint4 v = bias_raw[mat_bias16 ? c * 4 + i : 0];
+              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int y = 0; y < 4; ++y) {
-                  const float2 f = __fmul2_rn(unpack2<kBf16>(w[y]), make_float2(kLog2e, kLog2e));
-                  bb[8 * i + 2 * y] = f.x;
-                  bb[8 * i + 2 * y + 1] = f.y;
-                }
+              for (int y = 0; y < 4; ++y) {
+                const float2 f = __fmul2_rn(unpack2<kBf16>(w[y]), make_float2(kLog2e, kLog2e));
+                bb[8 * i + 2 * y] = f.x;
+                bb[8 * i + 2 * y + 1] = f.y;
               }
-            } else {
-              load_bias32<kBf16, mat_bias16 ? kBias16 : kBias32>(prm.ex, bias_row, k0n + c * 32, prm.Sk, bb);
             }
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) add_bias2(c, i, make_float2(bb[i], bb[i + 1]));
+          } else {
+            load_bias32<kBf16, mat_bias16 ? kBias16 : kBias32>(prm.ex, bias_row, k0n + c * 32, prm.Sk, bb);
           }
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) add_bias2(c, i, make_float2(bb[i], bb[i + 1]));
         }
         if (need_mask) {
 #pragma unroll
@@ -354,9 +348,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     };
 
     // prologue: scores of the first step; their row maximum is the first reference maximum
-    if constexpr (kExt != 0) {
-      if (vec_bias) stage_vec_bias(first);
-    }
+    if constexpr (vec_bias) stage_vec_bias(first);
     if constexpr (mat_bias16) fetch_mat_bias(first);
     mbar_wait(bar_s_full + 2 * s + first, 0, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
     tcgen05_fence_after_sync();
@@ -417,14 +409,12 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             if (first) {
               if (q & 1) mxb = max3(mxb, a, b); else mxa = max3(mxa, a, b);
             }
-            if constexpr (kExt != 0) {
+            if constexpr (has_drop) {
               // dropped elements leave the row sum untouched and enter P V as zeros; the factor
               // 1 / (1 - p) is applied once, to O, in the epilogue
-              if (has_drop) {
-                const uint32_t idx = drop_idx + static_cast<uint32_t>((kTight ? 0 : k0) + c * 32 + 2 * q);
-                if (dropout_hash(idx, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.x = 0.f;
-                if (dropout_hash(idx + 1u, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.y = 0.f;
-              }
+              const uint32_t idx = drop_idx + static_cast<uint32_t>((kTight ? 0 : k0) + c * 32 + 2 * q);
+              if (dropout_hash(idx, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.x = 0.f;
+              if (dropout_hash(idx + 1u, prm.ex.drop_seed) <= prm.ex.drop_threshold) x.y = 0.f;
             }
             pr[c][q] = pack2<kBf16>(x.x, x.y);
           }
@@ -454,13 +444,11 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // S of step t + 1 was issued when P of step t - 1 was handed over: complete by now as a
         // rule.  Its loads go out behind the P stores; the score registers are free, everything
         // of step t is in pr.
-        if constexpr (kExt != 0) {
-          if (vec_bias && u == 1) stage_vec_bias(t + 1);
-          if constexpr (mat_bias16) fetch_mat_bias(t + 1);
-          if (mat_bias && bias_row != nullptr && t + 2 < end) {
-            const int c0 = step_key(t + 2, first, key0);
-            prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0), up);
-          }
+        if (vec_bias && u == 1) stage_vec_bias(t + 1);
+        if constexpr (mat_bias16) fetch_mat_bias(t + 1);
+        if (mat_bias && bias_row != nullptr && t + 2 < end) {
+          const int c0 = step_key(t + 2, first, key0);
+          prefetch_bias(prm.ex, bias_row, c0, min(kStepN, prm.Sk - c0), up);
         }
         if (!s_next_ready)
           mbar_wait(bar_s_full + 2 * s + (u ^ 1), ((t + 1) >> 1) & 1, cta_abort, dstat, FO_STATUS_TIMEOUT_MMA);
@@ -501,7 +489,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tcgen05_fence_after_sync();
       const float l_run = s_final[s * 256 + r];
       const float m_run = s_final[s * 256 + 128 + r];
-      const float o_scale = (kExt != 0) ? prm.ex.drop_rescale : 1.f;
+      const float o_scale = prm.ex.drop_rescale;
       const float inv_l = (l_run > 0.f) ? o_scale / l_run : 0.f;
       const int row = (2 * pair + s) * kBlockM + r;
       const bool row_ok = row < prm.Sq;
