@@ -1,5 +1,5 @@
 """Sizes at which the kernel variants can go wrong: tile remainders, one to five query tiles (the
-barriers and buffers that alternate per tile), every combination of bias form and dropout."""
+barriers and buffers that alternate per tile), every compiled combination of bias form and dropout."""
 import pytest
 import torch
 
@@ -15,6 +15,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("D,code,bias_dtype,p", [
     (64, "matrix", torch.float32, 0.0), (64, "matrix", torch.bfloat16, 0.2), (64, None, None, 0.2),
     (64, "vector", torch.float32, 0.2), (40, "matrix", torch.bfloat16, 0.0), (128, "matrix", torch.float32, 0.2),
+    (64, "vector", torch.float32, 0.0), (64, None, None, 0.0), (128, "vector", torch.bfloat16, 0.0),
+    (128, "vector", torch.float32, 0.2), (128, "matrix", torch.bfloat16, 0.0), (128, None, None, 0.2),
+    (96, None, None, 0.0), (96, "vector", torch.float32, 0.0), (128, None, None, 0.0),
 ])
 def test_backward_bias_and_dropout_variants(cuda_device, Sq, Sk, causal, D, code, bias_dtype, p):
     B, H = 2, 2
