@@ -195,7 +195,8 @@ static int attn_bwd_impl(const void* q, const void* k, const void* v, const void
     else rc = bf16 ? launch_bwd<64, true, M>(tq, tk, tv, tdo, tdq, prm, s) : launch_bwd<64, false, M>(tq, tk, tv, tdo, tdq, prm, s);            \
     break;
   // head_dim 72 to 96 without bias and dropout: matmuls of width 96 in the 128-column tiles
-  // (B1 H48 Sq1000 Sk1531 D80 106 to 94 us, B1 H32 S4096 D96 causal 371 to 315); other sizes compute the zero columns of the next tile width.
+  // (B1 H48 Sq1000 Sk1531 D80 106 to 94 us, B1 H32 S4096 D96 causal 371 to 315); other sizes compute the
+  // zero columns of the next tile width.
   if (mode == 0 && D > 64 && D <= 96)
     rc = bf16 ? launch_bwd<128, true, 0, 96>(tq, tk, tv, tdo, tdq, prm, s) : launch_bwd<128, false, 0, 96>(tq, tk, tv, tdo, tdq, prm, s);
   else switch (mode) {

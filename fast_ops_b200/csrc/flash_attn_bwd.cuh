@@ -37,6 +37,8 @@
 // the fp32 buffer with tiled bulk reductions (cp.reduce.async.bulk.tensor).  Warp 12 issues the
 // MMAs, warp 13 the TMA loads, warp 14 brings LSE and delta of the next query tile into shared
 // memory (they vary along the columns, so every thread needs all 128 of them).
+// The wide form (BwdConfig::kWide) has sixteen compute warps, four threads per key row with 32 query
+// columns each (in the epilogue two for dK, two for dV), and the other roles in warps 16 to 22.
 #pragma once
 
 #include "flash_attn_common.cuh"
@@ -89,9 +91,13 @@ template <int D, int kExt>
 struct BwdConfig {
   // head_dim 64 with dropout or a matrix bias: sixteen compute warps (four threads per key row, 32
   // query columns each) instead of eight.  Hashing and fetching bias values are long chains per
-  // thread, and eight warps do not cover their latency: B2 H16 S2048 D64 with both 472 us with
-  // sixteen warps, 702 with eight (391 with sixteen since vector and matrix bias are compiled apart).  Without them eight warps are the faster form (B8 H12 S1024 D64
-  // causal 81 against 84 us), and at head_dim 128 the registers do not reach.
+  // thread, and eight warps do not cover their latency.  us, whole backward, B2 H16 S2048 / B8 H12 S1024
+  // causal / B32 H12 S128, before this form and with it: dropout 300 and 234 / 181 and 138 / 43 and 36;
+  // vector bias with dropout 317 and 235 / 188 and 139 / 44 and 37.  (A matrix bias also got its values
+  // 32 at a time: 2048 and 264 / 582 and 132 / 75 and 34, with dropout 2160 and 392 / 636 and 190 / 81 and
+  // 41.)  The compiler spills 24 to 84 bytes in all four.  Without dropout or a matrix bias eight warps are
+  // the faster form (B8 H12 S1024 D64 causal 81 against 84 us), and at head_dim 128 the registers do not
+  // reach.
   static constexpr bool kWide = D == 64 && (kExt & (kBwdDropout | kBwdMatBias)) != 0;
   static constexpr int kComputeWarps = kWide ? 16 : 8;
   static constexpr int kThreads = kComputeWarps * 32 + 256;
@@ -141,8 +147,9 @@ __device__ __forceinline__ void tmem_st_packed(uint32_t taddr, const uint32_t (&
 // 32 bias values (log2(e) * value) of one key and consecutive query rows: consecutive lanes hold
 // consecutive keys, so each load of a warp is one contiguous segment; all 32 are in flight
 // together (one load per element inside the exponential loop was waited for one by one: this
-// kernel took 2120 us at B2 H16 S2048 D64 with dropout, against 472).  `p` points at (first row, key) with key clamped into the row; rows past Sq read the
-// last row (their -LSE is -inf, or the caller replaces the value).
+// kernel took 2160 us at B2 H16 S2048 D64 with dropout, against 392).  `p` points at (first row, key)
+// with the key clamped into the row; rows past Sq (`rows_left` of them remain) are not loaded and give
+// 0: their -LSE is -inf, which makes P zero.
 template <bool kBf16>
 __device__ __forceinline__ void load_bias_rows32(const AttnExtras& ex, const uint8_t* p, int rows_left,
                                                  float (&out)[32]) {
@@ -572,9 +579,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       constexpr uint32_t idesc_q = make_idesc(kBf16, kBlockM, kMma, 1, 1);     // dQ: A M-major, B N-major
       constexpr uint32_t kBoxStep = kBoxBytes >> 4;
       // 16 queries per step; a thread's 16-bit results sit in the first half of its kCols columns
-      // Four steps go out per election: one election per matmul step made the whole kernel 1.5 to 2 %
-      // slower (B2 H32 S4096 D128 757 against 748 us), a branch per step 10 %.
-      // (kCols = 64: columns 0-31 and 64-95; kCols = 32: 0-15, 32-47, 64-79, 96-111)
+      // (kCols = 64: columns 0-31 and 64-95; kCols = 32: 0-15, 32-47, 64-79, 96-111).  Four steps go out
+      // per election: one election per matmul step made the whole backward 1 to 1.5 % slower
+      // (B2 H32 S4096 D128 causal 749 against 739 us), a branch per step 10 %.
       constexpr int kA1 = 8, kA2 = Cfg::kCols == 64 ? 16 : 32, kA3 = kA2 + 8;
       const uint32_t q_k = desc_lo(smem_u32(sQ), 16), do_k = desc_lo(smem_u32(sDO), 16);
       const uint32_t k_k = desc_lo(smem_u32(sK), 16), v_k = desc_lo(smem_u32(sV), 16);

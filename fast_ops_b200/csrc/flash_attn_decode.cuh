@@ -3,8 +3,9 @@
 //
 // Bound by memory: every key and value is used by one query row (or, when the heads share one K/V
 // head, by one row of each), so the 128-row tensor-core tiles of the other kernels would do 1/128
-// useful work, and one CTA per head leaves most SMs idle.  Here the keys of a head (or of kHeads heads that share
-// K and V) are split over the CTAs of a cluster and, inside a CTA, over its warps:
+// useful work, and one CTA per head leaves most SMs idle.  Here the keys of a
+// head (or of kHeads heads that share K and V) are split over the CTAs of a cluster and, inside a
+// CTA, over its warps:
 //   - a key's row is held by kLanes lanes, 16 bytes (8 elements) each; a warp takes kBatch rows
 //     per lane group and step, all of them in flight together (K of the next step is requested
 //     while V of this one is consumed);
@@ -15,8 +16,8 @@
 //   - warps combine through shared memory, CTAs of the cluster through distributed shared memory,
 //     so no workspace and no second launch.
 // Measured (one B200, us per launch, kernel alone; before = one 128-row tile per head):
-//   B4 H32 Sk4096 D128 bf16 54 -> 43 (41.6 at the measured copy rate); B1 H8 Sk32768 D128 354 -> 36;
-//   B2 H12 Sk19904 D64, one shared K/V head, 209 -> 15; B16 H32 Sk1000 D128, shared, 41 -> 21.
+//   B4 H32 Sk4096 D128 bf16 52 -> 42 (41.6 at the measured copy rate); B1 H8 Sk32768 D128 354 -> 36;
+//   B32 H40 Sk2000 D64, one shared K/V head, 143 -> 53; B16 H40 Sk1000 D128, shared, 50 -> 37.
 #pragma once
 
 #include <cooperative_groups.h>
