@@ -94,6 +94,12 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int n0 = (vis0 + kBlockN - 1) / kBlockN;
   const int n1 = (vis1 + kBlockN - 1) / kBlockN;
   const int T0 = 2 * n0, T1 = 2 * n1;  // T1 >= T0 >= 2
+  // The steps of a query tile are `first` to `end` - 1, two per key tile.  When the last key tile's upper
+  // half has no visible key (`odd`), one is left out (taken, with all its scores masked, it made 64 keys
+  // cost 38 us instead of 29 at B64 H12 D64, and 1088 keys 128 instead of 120 at B8 H16): going up the
+  // very last one, going down step 0, whose barrier phases are then completed at the set-up, so that
+  // step numbers stand for buffers and phases as ever.
+  const int odd0 = (vis0 + kStepN - 1) / kStepN & 1, odd1 = (vis1 + kStepN - 1) / kStepN & 1;
 
   if (tid == 0) {
     *cta_abort = 0;
@@ -108,8 +114,7 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       bias_first = load_bias1<kBf16>(prm.ex, p, 0);
       bias_last = load_bias1<kBf16>(prm.ex, p, vis0 - 1);
     }
-    *skip = *reinterpret_cast<volatile int*>(prm.device_status);
-    *ascending = bias_first - bias_last > kRescaleThreshold;
+    const int status = *reinterpret_cast<volatile int*>(prm.device_status);
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(bar_kv_full + i, 1);
@@ -126,20 +131,24 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       mbar_init(bar_final + s, 128);
       mbar_init(bar_o_done + s, 1);
     }
-    fence_mbar_init();
     prefetch_tensormap(&tm_q);
     prefetch_tensormap(&tm_k);
     prefetch_tensormap(&tm_v);
+    *skip = status;
+    const bool ascend = bias_first - bias_last > kRescaleThreshold;
+    *ascending = ascend;
+    for (int s = 0; s < 2; ++s)
+      if (!ascend && (s ? odd1 : odd0)) {  // the phases of a step 0 that is left out
+        mbar_arrive(bar_s_full + 2 * s);
+        mbar_arrive_n(bar_p_full + 2 * s, 256);
+        mbar_arrive_n(bar_corr + 2 * s, 128);
+        mbar_arrive(bar_o_full + s);
+      }
+    fence_mbar_init();
   }
   __syncthreads();
   if (*skip) return;  // another CTA already timed out: do nothing
   const bool up = *ascending != 0;
-  // The steps of a query tile are `first` to `last`, two per key tile.  When the last key tile's upper
-  // half has no visible key, one is left out (taken, with all its scores masked, it made 64 keys cost
-  // 38 us instead of 29 at B64 H12 D64, and 1088 keys 128 instead of 120 at B8 H16): going up the very
-  // last one, going down step 0, whose barrier phases are then completed in the set-up, so that step
-  // numbers stand for buffers and phases as ever.
-  const int odd0 = (vis0 + kStepN - 1) / kStepN & 1, odd1 = (vis1 + kStepN - 1) / kStepN & 1;
   const int first0 = up ? 0 : odd0, first1 = up ? 0 : odd1;
   const int end0 = up ? T0 - odd0 : T0, end1 = up ? T1 - odd1 : T1;
   // Tile 1 of the pair has up to two steps more than tile 0, those next to the diagonal: going down
@@ -171,17 +180,6 @@ attn_fwd_ws64r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tma_load_4d(sQ + s * kTileBytes + c * kBoxBytes, &tm_q, bar_q_full, c * kBoxCols,
                     (2 * pair + s) * kBlockM, h, b);
     for (int i = 0; i < first_fill; ++i) load_kv(i);
-  }
-  // the phases of a step 0 that is left out
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    if (!(s ? first1 : first0)) continue;
-    if (warp >> 2 == s) mbar_arrive(bar_corr + 2 * s);
-    if (warp >> 2 == s || warp >> 2 == 2) mbar_arrive(bar_p_full + 2 * s);
-    if (warp == (s ? 14 : 12) && lane == 0) {
-      mbar_arrive(bar_s_full + 2 * s);
-      mbar_arrive(bar_o_full + s);
-    }
   }
   if (warp == 12) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
